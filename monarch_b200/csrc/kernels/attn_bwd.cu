@@ -15,15 +15,23 @@
 // buffer and no transposed copy of dS in shared memory: every operand is either a TMA tile
 // or lives in TMEM.  Accumulators never leave TMEM until the epilogue.
 //
-// Both kernels step through their inner dimension 64 rows at a time with two sets of
-// (S, dP) accumulator columns: while the eight compute warps turn set t&1 into bf16
-// operands, the tensor pipe already runs S and dP of step t+1 into the other set, and the
-// accumulating MMAs of step t follow as soon as its operands are written.
+// Both kernels step through their inner dimension 128 rows at a time.  A 128x128x128 MMA with
+// both operands in shared memory reads 64 KB in the 512 cycles the tensor pipe needs for it
+// (measured: 514 cycles); a 128x64x128 one still reads 48 KB in 256 cycles of math and takes
+// 386, so 64-row steps made the scores a third more expensive.  With 128-row steps TMEM is full
+// (dK, dV, S, dP: 4 x 128 columns at hd 128), and the overlap of math and exponentials comes
+// from the order in which the MMA warp issues, not from a second set of accumulators:
+//   dK/dV:  dV(t)  S(t+1)  dK(t)  dP(t+1) ...    P(t+1) is computed under dK(t) and dP(t+1),
+//                                                dS(t+1) under dV(t+1) and S(t+2)
+//   dQ:     S(t+1) dP(t+1) dQ(t) ...             (dP has two buffers here, S is free again as
+//                                                soon as the warps hold it in registers)
+// B1 S8192 32q/8kv hd128: dK/dV 1361 -> 853 us, dQ 1223 -> 616 us against the 64-row steps;
+// B2 S4096 32q/8kv hd64: 551 -> 383 us and 518 -> 281 us.
 //
 // Warp roles (576 threads): 0 TMA producer, 1 MMA issuer, 2-17 compute/epilogue; warps w,
-// w+4, w+8, w+12 share a TMEM lane quadrant and split the 64 columns of a set in quarters
+// w+4, w+8, w+12 share a TMEM lane quadrant and split the 128 columns of a tile in quarters
 // (four warps per scheduler hide the TMEM load latency of each other).  The bf16 operand of
-// quarter c is written at columns [16c, 16c+8) of the fp32 columns it replaces, so no warp
+// quarter c is written at columns [32c, 32c+16) of the fp32 columns it replaces, so no warp
 // overwrites columns another warp still has to read.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -82,26 +90,6 @@ __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------------ dK, dV
-constexpr int AB_SUB = 64;       // rows of the streamed operand per step
-constexpr int AB_STAGES = 4;
-
-template <int HD>
-struct DkvSmem {
-  static constexpr int kTile = AB_T * HD * 2;          // K, V (resident)
-  static constexpr int kSub = AB_SUB * HD * 2;         // Q or dO sub-tile
-  static constexpr int kStage = 2 * kSub + 1024;       // Q, dO, lse[64], delta[64] (+pad)
-  static constexpr int kData = 2 * kTile + AB_STAGES * kStage;
-  static constexpr int kTotal = kData + 1024 + 256;
-};
-
-struct DkvBars {
-  uint64_t kv_full;
-  uint64_t qdo_full[AB_STAGES], qdo_empty[AB_STAGES];
-  uint64_t sdp_full[2], pds_ready[2], acc_done;
-  uint32_t tmem_base;
-  volatile int abort_word;
-};
-
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes,
                                              uint64_t* bar) {
   asm volatile(
@@ -110,22 +98,79 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
       : "memory");
 }
 
+// The operand that the last MMA of a step still reads has three stages (its buffer comes free
+// only two MMAs before the next tile in it is needed), the other one two.
+constexpr int AB_ST3 = 3;
+constexpr int AB_ST2 = 2;
+
+// Both kernels: two resident tiles, a ring of three and a ring of two tiles.  With hd 128 that
+// is 224 KB, which leaves no room to align the base by hand: the dynamic shared memory itself
+// is declared 1024-byte aligned (no static shared memory in these kernels).
+template <int HD>
+struct AbSmem {
+  static constexpr int kTile = AB_T * HD * 2;
+  static constexpr int kRowBytes = AB_T * 4;       // lse or delta of 128 query rows
+  static constexpr int kData = (2 + AB_ST3 + AB_ST2) * kTile;
+  static constexpr int kTotal = kData + AB_ST2 * 2 * kRowBytes + 256;
+  static_assert(kTotal <= 232448, "more than 227 KB of shared memory");
+};
+
+struct DkvBars {
+  uint64_t kv_full;
+  uint64_t q_full[AB_ST3], q_empty[AB_ST3];
+  uint64_t do_full[AB_ST2], do_empty[AB_ST2];
+  uint64_t ld_full[AB_ST2], ld_empty[AB_ST2];
+  uint64_t s_full, dp_full, p_ready, ds_ready, acc_done;
+  uint32_t tmem_base;
+  volatile int abort_word;
+};
+static_assert(sizeof(DkvBars) <= 256, "barriers outgrew their space");
+
+// A 128-row tile of `HD` columns as 64-column slices
+template <int HD>
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, uint64_t* bar,
+                                          int col, int row) {
+#pragma unroll
+  for (int c = 0; c < HD / 64; ++c)
+    tma_load_2d(dst + c * (AB_T * 128), m, bar, col + c * 64, row);
+}
+// D[128, 128] = A B^T over HD, both tiles K-major in shared memory
+template <int HD>
+__device__ __forceinline__ void mma_scores(uint32_t d_tmem, uint32_t sa, uint32_t sb) {
+  constexpr uint32_t idesc = umma_idesc_bf16(AB_T, AB_T, 0, 0);
+#pragma unroll
+  for (int kk = 0; kk < HD / 16; ++kk) {
+    const uint32_t off = (kk / 4) * (AB_T * 128) + (kk % 4) * 32;
+    umma_f16(d_tmem, umma_smem_desc_sw128(sa + off, 16, 1024),
+             umma_smem_desc_sw128(sb + off, 16, 1024), idesc, kk > 0 ? 1u : 0u);
+  }
+}
+// D[128, HD] (+)= A B over 128 rows: A bf16 in TMEM (quarters of 16 columns every 32), B MN-major
+template <int HD>
+__device__ __forceinline__ void mma_grad(uint32_t d_tmem, uint32_t a_tmem, uint32_t sb,
+                                         bool accumulate) {
+  constexpr uint32_t idesc = umma_idesc_bf16(AB_T, HD, 0, 1);
+#pragma unroll
+  for (int kk = 0; kk < AB_T / 16; ++kk)
+    umma_f16_ts(d_tmem, a_tmem + (kk >> 1) * 32 + (kk & 1) * 8,
+                umma_smem_desc_sw128(sb + kk * 2048, AB_T * 128, 1024), idesc,
+                (accumulate || kk > 0) ? 1u : 0u);
+}
+
 template <int HD>
 __global__ void __launch_bounds__(AB_THREADS, 1)
-    attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ,    // box 64 x 64 rows
-                        const __grid_constant__ CUtensorMap tmK,    // box 64 x 128 rows
+    attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ,
+                        const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV,
-                        const __grid_constant__ CUtensorMap tmDO,   // box 64 x 64 rows
-                        const AttBwdParams p) {
-  using SM = DkvSmem<HD>;
-  constexpr int NCH = HD / 64;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+                        const __grid_constant__ CUtensorMap tmDO, const AttBwdParams p) {
+  using SM = AbSmem<HD>;
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
   uint8_t* sV = sK + SM::kTile;
-  uint8_t* sStage = sV + SM::kTile;
-  DkvBars* bars = reinterpret_cast<DkvBars*>(smem + SM::kData);
+  uint8_t* sQ = sV + SM::kTile;                 // [AB_ST3]
+  uint8_t* sDO = sQ + AB_ST3 * SM::kTile;       // [AB_ST2]
+  float* sLD = reinterpret_cast<float*>(smem + SM::kData);  // [AB_ST2] x {lse[128], delta[128]}
+  DkvBars* bars = reinterpret_cast<DkvBars*>(smem + SM::kData + AB_ST2 * 2 * SM::kRowBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -138,20 +183,26 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   const int kv_head = hb % p.Hkv;
   const int b = hb / p.Hkv;
   const int group = p.Hq / p.Hkv;
-  const int nq = 2 * (n_blk - j);    // 64-row query sub-blocks at or below the diagonal
+  const int nq = n_blk - j;          // query blocks at or below the diagonal
   const int nsteps = group * nq;
   const int row_base = b * p.S;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->kv_full, 1);
-    for (int s = 0; s < AB_STAGES; ++s) {
-      mbar_init(&bars->qdo_full[s], 1);
-      mbar_init(&bars->qdo_empty[s], 1);
+    for (int s = 0; s < AB_ST3; ++s) {
+      mbar_init(&bars->q_full[s], 1);
+      mbar_init(&bars->q_empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&bars->sdp_full[s], 1);
-      mbar_init(&bars->pds_ready[s], 16);
+    for (int s = 0; s < AB_ST2; ++s) {
+      mbar_init(&bars->do_full[s], 1);
+      mbar_init(&bars->do_empty[s], 1);
+      mbar_init(&bars->ld_full[s], 1);
+      mbar_init(&bars->ld_empty[s], 1);
     }
+    mbar_init(&bars->s_full, 1);
+    mbar_init(&bars->dp_full, 1);
+    mbar_init(&bars->p_ready, 16);
+    mbar_init(&bars->ds_ready, 16);
     mbar_init(&bars->acc_done, 1);
     bars->abort_word = 0;
     mbar_fence_init();
@@ -165,153 +216,173 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile int* abort_word = &bars->abort_word;
-  // TMEM columns: set s: S^T/P^T at s*128, dP^T/dS^T at s*128 + 64; dV at 256, dK at 256 + HD
-  constexpr uint32_t kColDV = 256, kColDK = 256 + HD;
+  // TMEM columns: S^T/P^T at 0, dP^T/dS^T at 128, dV at 256, dK at 256 + HD
+  constexpr uint32_t kColDP = 128, kColDV = 256, kColDK = 256 + HD;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
       tma_prefetch_desc(&tmDO);
       mbar_expect_tx(&bars->kv_full, 2 * SM::kTile);
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        tma_load_2d(sK + c * (AB_T * 128), &tmK, &bars->kv_full, kv_head * HD + c * 64,
-                    row_base + j * AB_T);
-        tma_load_2d(sV + c * (AB_T * 128), &tmV, &bars->kv_full, kv_head * HD + c * 64,
-                    row_base + j * AB_T);
-      }
+      load_tile<HD>(sK, &tmK, &bars->kv_full, kv_head * HD, row_base + j * AB_T);
+      int h = kv_head * group, qb = j;   // head and query block of step t
       for (int t = 0; t < nsteps; ++t) {
-        const int st = t % AB_STAGES;
-        if (!mbar_wait(&bars->qdo_empty[st], ((uint32_t)(t / AB_STAGES) & 1) ^ 1, abort_word,
-                       p.status))
-          break;
-        const int h = kv_head * group + t / nq;
-        const int q0 = (2 * j + t % nq) * AB_SUB;   // first query row of this sub-block
-        uint8_t* sq = sStage + st * SM::kStage;
-        uint8_t* sdo = sq + SM::kSub;
-        float* sl = reinterpret_cast<float*>(sdo + SM::kSub);
-        mbar_expect_tx(&bars->qdo_full[st], 2 * SM::kSub + 512);
-#pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          tma_load_2d(sq + c * (AB_SUB * 128), &tmQ, &bars->qdo_full[st], h * HD + c * 64,
-                      row_base + q0);
-          tma_load_2d(sdo + c * (AB_SUB * 128), &tmDO, &bars->qdo_full[st], h * HD + c * 64,
-                      row_base + q0);
+        const int s3 = t % AB_ST3, s2 = t % AB_ST2;
+        const uint32_t ph3 = ((uint32_t)(t / AB_ST3) & 1) ^ 1;
+        const uint32_t ph2 = ((uint32_t)(t / AB_ST2) & 1) ^ 1;
+        if (!mbar_wait(&bars->q_empty[s3], ph3, abort_word, p.status)) break;
+        mbar_expect_tx(&bars->q_full[s3], SM::kTile);
+        load_tile<HD>(sQ + s3 * SM::kTile, &tmQ, &bars->q_full[s3], h * HD, row_base + qb * AB_T);
+        if (t == 0) load_tile<HD>(sV, &tmV, &bars->kv_full, kv_head * HD, row_base + j * AB_T);
+        if (!mbar_wait(&bars->do_empty[s2], ph2, abort_word, p.status)) break;
+        mbar_expect_tx(&bars->do_full[s2], SM::kTile);
+        load_tile<HD>(sDO + s2 * SM::kTile, &tmDO, &bars->do_full[s2], h * HD,
+                      row_base + qb * AB_T);
+        if (!mbar_wait(&bars->ld_empty[s2], ph2, abort_word, p.status)) break;
+        mbar_expect_tx(&bars->ld_full[s2], 2 * SM::kRowBytes);
+        const size_t lrow = ((size_t)b * p.Hq + h) * p.S + (size_t)qb * AB_T;
+        bulk_load_1d(sLD + s2 * 2 * AB_T, p.lse + lrow, SM::kRowBytes, &bars->ld_full[s2]);
+        bulk_load_1d(sLD + s2 * 2 * AB_T + AB_T, p.delta + lrow, SM::kRowBytes,
+                     &bars->ld_full[s2]);
+        if (++qb == n_blk) {
+          qb = j;
+          ++h;
         }
-        const size_t lrow = ((size_t)b * p.Hq + h) * p.S + (size_t)q0;
-        bulk_load_1d(sl, p.lse + lrow, 256, &bars->qdo_full[st]);
-        bulk_load_1d(sl + 64, p.delta + lrow, 256, &bars->qdo_full[st]);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_ss = umma_idesc_bf16(AB_T, AB_SUB, 0, 0);
-      constexpr uint32_t idesc_ts = umma_idesc_bf16(AB_T, HD, 0, 1);
-      bool ok = mbar_wait(&bars->kv_full, 0, abort_word, p.status);
-      tc_fence_after();
+    if (elect_one()) {
       const uint32_t sk = smem_u32(sK), sv = smem_u32(sV);
-      // S^T and dP^T of step t into accumulator set t&1
-      auto issue_sdp = [&](int t) -> bool {
-        const int st = t % AB_STAGES;
-        if (!mbar_wait(&bars->qdo_full[st], (uint32_t)(t / AB_STAGES) & 1, abort_word, p.status))
-          return false;
+      const uint32_t sq = smem_u32(sQ), sdo = smem_u32(sDO);
+      bool ok = mbar_wait(&bars->kv_full, 0, abort_word, p.status) &&
+                mbar_wait(&bars->q_full[0], 0, abort_word, p.status);
+      if (ok) {
         tc_fence_after();
-        const uint32_t sq = smem_u32(sStage + st * SM::kStage);
-        const uint32_t sdo = sq + SM::kSub;
-        const uint32_t c_st = tmem_base + (t & 1) * 128, c_dp = c_st + 64;
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t offk = (kk / 4) * (AB_T * 128) + (kk % 4) * 32;
-          const uint32_t offq = (kk / 4) * (AB_SUB * 128) + (kk % 4) * 32;
-          umma_f16(c_st, umma_smem_desc_sw128(sk + offk, 16, 1024),
-                   umma_smem_desc_sw128(sq + offq, 16, 1024), idesc_ss, kk > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t offk = (kk / 4) * (AB_T * 128) + (kk % 4) * 32;
-          const uint32_t offq = (kk / 4) * (AB_SUB * 128) + (kk % 4) * 32;
-          umma_f16(c_dp, umma_smem_desc_sw128(sv + offk, 16, 1024),
-                   umma_smem_desc_sw128(sdo + offq, 16, 1024), idesc_ss, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&bars->sdp_full[t & 1]);
-        return true;
-      };
-      if (ok && nsteps > 0) ok = issue_sdp(0);
+        mma_scores<HD>(tmem_base, sk, sq);
+        umma_commit(&bars->s_full);
+        ok = mbar_wait(&bars->do_full[0], 0, abort_word, p.status);
+      }
+      if (ok) {
+        tc_fence_after();
+        mma_scores<HD>(tmem_base + kColDP, sv, sdo);
+        umma_commit(&bars->dp_full);
+      }
       for (int t = 0; ok && t < nsteps; ++t) {
-        if (t + 1 < nsteps) {
-          ok = issue_sdp(t + 1);   // runs on the tensor pipe while the warps work on step t
-          if (!ok) break;
-        }
-        ok = mbar_wait(&bars->pds_ready[t & 1], (uint32_t)(t >> 1) & 1, abort_word, p.status);
+        const int q3 = t % AB_ST3, d2 = t % AB_ST2;
+        const int nq3 = (t + 1) % AB_ST3, nd2 = (t + 1) % AB_ST2;
+        const uint32_t par = (uint32_t)t & 1;
+        const bool more = t + 1 < nsteps;
+        ok = mbar_wait(&bars->p_ready, par, abort_word, p.status);
         if (!ok) break;
         tc_fence_after();
-        const int st = t % AB_STAGES;
-        const uint32_t sq = smem_u32(sStage + st * SM::kStage);
-        const uint32_t sdo = sq + SM::kSub;
-        const uint32_t c_st = tmem_base + (t & 1) * 128, c_dp = c_st + 64;
-#pragma unroll
-        for (int kk = 0; kk < AB_SUB / 16; ++kk) {
-          const uint32_t a_col = kk * 16;  // bf16 quarter kk sits at columns [16kk, 16kk+8)
-          umma_f16_ts(tmem_base + kColDV, c_st + a_col,
-                      umma_smem_desc_sw128(sdo + kk * 2048, AB_SUB * 128, 1024), idesc_ts,
-                      (t > 0 || kk > 0) ? 1u : 0u);
+        mma_grad<HD>(tmem_base + kColDV, tmem_base, sdo + d2 * SM::kTile, t > 0);
+        umma_commit(&bars->do_empty[d2]);
+        if (more) {   // overwrites P(t): ordered behind dV(t) on the tensor pipe
+          ok = mbar_wait(&bars->q_full[nq3], (uint32_t)((t + 1) / AB_ST3) & 1, abort_word,
+                         p.status);
+          if (!ok) break;
+          tc_fence_after();
+          mma_scores<HD>(tmem_base, sk, sq + nq3 * SM::kTile);
+          umma_commit(&bars->s_full);
         }
-#pragma unroll
-        for (int kk = 0; kk < AB_SUB / 16; ++kk) {
-          const uint32_t a_col = kk * 16;
-          umma_f16_ts(tmem_base + kColDK, c_dp + a_col,
-                      umma_smem_desc_sw128(sq + kk * 2048, AB_SUB * 128, 1024), idesc_ts,
-                      (t > 0 || kk > 0) ? 1u : 0u);
+        ok = mbar_wait(&bars->ds_ready, par, abort_word, p.status);
+        if (!ok) break;
+        tc_fence_after();
+        mma_grad<HD>(tmem_base + kColDK, tmem_base + kColDP, sq + q3 * SM::kTile, t > 0);
+        umma_commit(&bars->q_empty[q3]);
+        umma_commit(&bars->ld_empty[d2]);   // lse and delta of step t were read before dS(t)
+        if (more) {
+          ok = mbar_wait(&bars->do_full[nd2], (uint32_t)((t + 1) / AB_ST2) & 1, abort_word,
+                         p.status);
+          if (!ok) break;
+          tc_fence_after();
+          mma_scores<HD>(tmem_base + kColDP, sv, sdo + nd2 * SM::kTile);
+          umma_commit(&bars->dp_full);
         }
-        umma_commit(&bars->qdo_empty[st]);
       }
       if (ok) umma_commit(&bars->acc_done);
     }
   } else {
     const int quad = warp & 3;
-    const int part = (warp - 2) >> 2;  // quarter of the 64 columns this warp converts
+    const int part = (warp - 2) >> 2;  // quarter of the 128 columns this warp converts
     const int r = quad * 32 + lane;    // kv row inside the block
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    const uint32_t t_st = tmem_base + lane_off + part * 32;
+    const uint32_t t_dp = t_st + kColDP;
+    const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    const uint64_t nlog2e = pack_f32x2(-kLog2e, -kLog2e);
+    const uint64_t neg1 = pack_f32x2(-1.f, -1.f);
     bool ok = true;
+    int sub = 0;                       // query block of this step relative to the diagonal
     for (int t = 0; t < nsteps; ++t) {
-      ok = mbar_wait(&bars->sdp_full[t & 1], (uint32_t)(t >> 1) & 1, abort_word, p.status);
+      const int s2 = t % AB_ST2;
+      const uint32_t par = (uint32_t)t & 1;
+      ok = mbar_wait(&bars->ld_full[s2], (uint32_t)(t / AB_ST2) & 1, abort_word, p.status);
+      if (!ok) break;
+      const float* sl = sLD + s2 * 2 * AB_T + part * 32;
+      ok = mbar_wait(&bars->s_full, par, abort_word, p.status);
       if (!ok) break;
       tc_fence_after();
-      const int st = t % AB_STAGES;
-      const float* sl = reinterpret_cast<const float*>(sStage + st * SM::kStage + 2 * SM::kSub);
-      const uint32_t t_st = tmem_base + (t & 1) * 128 + lane_off + part * 16;
-      const uint32_t t_dp = t_st + 64;
-      // query sub-blocks 2j and 2j+1 overlap the diagonal of kv block j
-      const int sub = t % nq;
-      const int q_rel = sub * AB_SUB + part * 16;  // first query of this warp, rel. to kv row 0
-      uint32_t sv[16], dv[16];
-      tmem_ld_32x32b_x16(t_st, sv);
-      tmem_ld_32x32b_x16(t_dp, dv);
+      uint32_t sv[32];
+      tmem_ld_32x32b_x32(t_st, sv);
       tmem_ld_wait();
-      uint32_t pp[8], ds[8];
+      uint32_t pk[16];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float2 l2 = *reinterpret_cast<const float2*>(sl + part * 16 + 2 * i);
-        const float2 d2 = *reinterpret_cast<const float2*>(sl + 64 + part * 16 + 2 * i);
-        float p0 = ex2_approx(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2, -l2.x * kLog2e));
-        float p1 = ex2_approx(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2, -l2.y * kLog2e));
-        if (sub < 2) {
-          if (q_rel + 2 * i < r) p0 = 0.f;      // query position before the key position
-          if (q_rel + 2 * i + 1 < r) p1 = 0.f;
+        const float4 l4 = *reinterpret_cast<const float4*>(sl + 4 * i);
+        const float2 e0 = unpack_f32x2(
+            fma_f32x2(pack_f32x2(__uint_as_float(sv[4 * i]), __uint_as_float(sv[4 * i + 1])), c2,
+                      mul_f32x2(pack_f32x2(l4.x, l4.y), nlog2e)));
+        const float2 e1 = unpack_f32x2(
+            fma_f32x2(pack_f32x2(__uint_as_float(sv[4 * i + 2]), __uint_as_float(sv[4 * i + 3])),
+                      c2, mul_f32x2(pack_f32x2(l4.z, l4.w), nlog2e)));
+        float pv[4] = {ex2_approx(e0.x), ex2_approx(e0.y), ex2_approx(e1.x), ex2_approx(e1.y)};
+        if (sub == 0) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (part * 32 + 4 * i + e < r) pv[e] = 0.f;  // query before the key position
         }
-        const float s0 = p0 * (__uint_as_float(dv[2 * i]) - d2.x);
-        const float s1 = p1 * (__uint_as_float(dv[2 * i + 1]) - d2.y);
-        pp[i] = pack_bf16x2(p0, p1);
-        ds[i] = pack_bf16x2(s0, s1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sv[4 * i + e] = __float_as_uint(pv[e]);
+        pk[2 * i] = pack_bf16x2(pv[0], pv[1]);
+        pk[2 * i + 1] = pack_bf16x2(pv[2], pv[3]);
       }
-      tmem_st_32x32b_x8(t_st, pp);
-      tmem_st_32x32b_x8(t_dp, ds);
+      tmem_st_32x32b_x16(t_st, pk);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->pds_ready[t & 1]);
+      if (lane == 0) mbar_arrive(&bars->p_ready);
+      ok = mbar_wait(&bars->dp_full, par, abort_word, p.status);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t dv[32];
+      tmem_ld_32x32b_x32(t_dp, dv);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 d4 = *reinterpret_cast<const float4*>(sl + AB_T + 4 * i);
+        // dP - delta as fma(delta, -1, dP): one rounding, like the subtraction
+        const uint64_t a0 = fma_f32x2(
+            pack_f32x2(d4.x, d4.y), neg1,
+            pack_f32x2(__uint_as_float(dv[4 * i]), __uint_as_float(dv[4 * i + 1])));
+        const uint64_t a1 = fma_f32x2(
+            pack_f32x2(d4.z, d4.w), neg1,
+            pack_f32x2(__uint_as_float(dv[4 * i + 2]), __uint_as_float(dv[4 * i + 3])));
+        const float2 x0 = unpack_f32x2(mul_f32x2(
+            a0, pack_f32x2(__uint_as_float(sv[4 * i]), __uint_as_float(sv[4 * i + 1]))));
+        const float2 x1 = unpack_f32x2(mul_f32x2(
+            a1, pack_f32x2(__uint_as_float(sv[4 * i + 2]), __uint_as_float(sv[4 * i + 3]))));
+        pk[2 * i] = pack_bf16x2(x0.x, x0.y);
+        pk[2 * i + 1] = pack_bf16x2(x1.x, x1.y);
+      }
+      tmem_st_32x32b_x16(t_dp, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->ds_ready);
+      if (++sub == nq) sub = 0;
     }
     if (ok) ok = mbar_wait(&bars->acc_done, 0, abort_word, p.status);
     if (ok) {
@@ -359,38 +430,28 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
 }
 
 // ----------------------------------------------------------------------------- dQ
-template <int HD>
-struct DqSmem {
-  static constexpr int kTile = AB_T * HD * 2;      // Q, dO (resident)
-  static constexpr int kSub = AB_SUB * HD * 2;     // K or V sub-tile
-  static constexpr int kStage = 2 * kSub;
-  static constexpr int kData = 2 * kTile + AB_STAGES * kStage;
-  static constexpr int kTotal = kData + 1024 + 256;
-};
-
 struct DqBars {
   uint64_t qdo_full;
-  uint64_t kv_full[AB_STAGES], kv_empty[AB_STAGES];
-  uint64_t sdp_full[2], ds_ready[2], acc_done;
+  uint64_t k_full[AB_ST3], k_empty[AB_ST3];
+  uint64_t v_full[AB_ST2], v_empty[AB_ST2];
+  uint64_t s_full, s_free, dp_full[2], ds_ready[2], acc_done;
   uint32_t tmem_base;
   volatile int abort_word;
 };
+static_assert(sizeof(DqBars) <= 256, "barriers outgrew their space");
 
 template <int HD>
 __global__ void __launch_bounds__(AB_THREADS, 1)
-    attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ,    // box 64 x 128 rows
-                       const __grid_constant__ CUtensorMap tmK,    // box 64 x 64 rows
+    attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ,
+                       const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV,
-                       const __grid_constant__ CUtensorMap tmDO,   // box 64 x 128 rows
-                       const AttBwdParams p) {
-  using SM = DqSmem<HD>;
-  constexpr int NCH = HD / 64;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+                       const __grid_constant__ CUtensorMap tmDO, const AttBwdParams p) {
+  using SM = AbSmem<HD>;
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;
   uint8_t* sDO = sQ + SM::kTile;
-  uint8_t* sKV = sDO + SM::kTile;  // [stages] x {K sub-tile, V sub-tile}
+  uint8_t* sK = sDO + SM::kTile;             // [AB_ST3]
+  uint8_t* sV = sK + AB_ST3 * SM::kTile;     // [AB_ST2]
   DqBars* bars = reinterpret_cast<DqBars*>(smem + SM::kData);
 
   const int warp = threadIdx.x >> 5;
@@ -401,18 +462,22 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   const int b = blockIdx.z;
   const int kv_head = h / (p.Hq / p.Hkv);
   const int row_base = b * p.S;
-  const int nsteps = 2 * (i + 1);             // 64-row kv sub-blocks up to the diagonal
+  const int nsteps = i + 1;                   // kv blocks up to the diagonal
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->qdo_full, 1);
-    for (int s = 0; s < AB_STAGES; ++s) {
-      mbar_init(&bars->kv_full[s], 1);
-      mbar_init(&bars->kv_empty[s], 1);
+    for (int s = 0; s < AB_ST3; ++s) {
+      mbar_init(&bars->k_full[s], 1);
+      mbar_init(&bars->k_empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&bars->sdp_full[s], 1);
+      mbar_init(&bars->v_full[s], 1);
+      mbar_init(&bars->v_empty[s], 1);
+      mbar_init(&bars->dp_full[s], 1);
       mbar_init(&bars->ds_ready[s], 16);
     }
+    mbar_init(&bars->s_full, 1);
+    mbar_init(&bars->s_free, 16);
     mbar_init(&bars->acc_done, 1);
     bars->abort_word = 0;
     mbar_fence_init();
@@ -426,70 +491,54 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile int* abort_word = &bars->abort_word;
-  // TMEM columns: set s: S at s*128, dP/dS at s*128 + 64; dQ at 256
-  constexpr uint32_t kColDQ = 256;
+  // TMEM columns: S at 0, dP/dS of step t at 128 + (t&1)*128, dQ at 384
+  constexpr uint32_t kColDP = 128, kColDQ = 384;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
       tma_prefetch_desc(&tmDO);
       mbar_expect_tx(&bars->qdo_full, 2 * SM::kTile);
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        tma_load_2d(sQ + c * (AB_T * 128), &tmQ, &bars->qdo_full, h * HD + c * 64,
-                    row_base + i * AB_T);
-        tma_load_2d(sDO + c * (AB_T * 128), &tmDO, &bars->qdo_full, h * HD + c * 64,
-                    row_base + i * AB_T);
-      }
+      load_tile<HD>(sQ, &tmQ, &bars->qdo_full, h * HD, row_base + i * AB_T);
       for (int t = 0; t < nsteps; ++t) {
-        const int st = t % AB_STAGES;
-        if (!mbar_wait(&bars->kv_empty[st], ((uint32_t)(t / AB_STAGES) & 1) ^ 1, abort_word,
+        const int s3 = t % AB_ST3, s2 = t % AB_ST2;
+        if (!mbar_wait(&bars->k_empty[s3], ((uint32_t)(t / AB_ST3) & 1) ^ 1, abort_word,
                        p.status))
           break;
-        uint8_t* sk = sKV + st * SM::kStage;
-        uint8_t* sv = sk + SM::kSub;
-        mbar_expect_tx(&bars->kv_full[st], 2 * SM::kSub);
-#pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          tma_load_2d(sk + c * (AB_SUB * 128), &tmK, &bars->kv_full[st], kv_head * HD + c * 64,
-                      row_base + t * AB_SUB);
-          tma_load_2d(sv + c * (AB_SUB * 128), &tmV, &bars->kv_full[st], kv_head * HD + c * 64,
-                      row_base + t * AB_SUB);
-        }
+        mbar_expect_tx(&bars->k_full[s3], SM::kTile);
+        load_tile<HD>(sK + s3 * SM::kTile, &tmK, &bars->k_full[s3], kv_head * HD,
+                      row_base + t * AB_T);
+        if (t == 0) load_tile<HD>(sDO, &tmDO, &bars->qdo_full, h * HD, row_base + i * AB_T);
+        if (!mbar_wait(&bars->v_empty[s2], ((uint32_t)(t / AB_ST2) & 1) ^ 1, abort_word,
+                       p.status))
+          break;
+        mbar_expect_tx(&bars->v_full[s2], SM::kTile);
+        load_tile<HD>(sV + s2 * SM::kTile, &tmV, &bars->v_full[s2], kv_head * HD,
+                      row_base + t * AB_T);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_ss = umma_idesc_bf16(AB_T, AB_SUB, 0, 0);
-      constexpr uint32_t idesc_ts = umma_idesc_bf16(AB_T, HD, 0, 1);
-      bool ok = mbar_wait(&bars->qdo_full, 0, abort_word, p.status);
-      tc_fence_after();
+    if (elect_one()) {
       const uint32_t sq = smem_u32(sQ), sdo = smem_u32(sDO);
+      const uint32_t sk = smem_u32(sK), sv = smem_u32(sV);
+      bool ok = mbar_wait(&bars->qdo_full, 0, abort_word, p.status);
+      // S and dP of step t; S(t-1) must have been read, dP's buffer was last read by dQ(t-2)
       auto issue_sdp = [&](int t) -> bool {
-        const int st = t % AB_STAGES;
-        if (!mbar_wait(&bars->kv_full[st], (uint32_t)(t / AB_STAGES) & 1, abort_word, p.status))
+        const int s3 = t % AB_ST3, s2 = t % AB_ST2;
+        if (!mbar_wait(&bars->k_full[s3], (uint32_t)(t / AB_ST3) & 1, abort_word, p.status) ||
+            !mbar_wait(&bars->s_free, ((uint32_t)t & 1) ^ 1, abort_word, p.status))
           return false;
         tc_fence_after();
-        const uint32_t sk = smem_u32(sKV + st * SM::kStage);
-        const uint32_t sv = sk + SM::kSub;
-        const uint32_t c_s = tmem_base + (t & 1) * 128, c_dp = c_s + 64;
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t offq = (kk / 4) * (AB_T * 128) + (kk % 4) * 32;
-          const uint32_t offk = (kk / 4) * (AB_SUB * 128) + (kk % 4) * 32;
-          umma_f16(c_s, umma_smem_desc_sw128(sq + offq, 16, 1024),
-                   umma_smem_desc_sw128(sk + offk, 16, 1024), idesc_ss, kk > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t offq = (kk / 4) * (AB_T * 128) + (kk % 4) * 32;
-          const uint32_t offk = (kk / 4) * (AB_SUB * 128) + (kk % 4) * 32;
-          umma_f16(c_dp, umma_smem_desc_sw128(sdo + offq, 16, 1024),
-                   umma_smem_desc_sw128(sv + offk, 16, 1024), idesc_ss, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&bars->sdp_full[t & 1]);
+        mma_scores<HD>(tmem_base, sq, sk + s3 * SM::kTile);
+        umma_commit(&bars->s_full);
+        if (!mbar_wait(&bars->v_full[s2], (uint32_t)(t / AB_ST2) & 1, abort_word, p.status))
+          return false;
+        tc_fence_after();
+        mma_scores<HD>(tmem_base + kColDP + (t & 1) * 128, sdo, sv + s2 * SM::kTile);
+        umma_commit(&bars->dp_full[t & 1]);
+        umma_commit(&bars->v_empty[s2]);
         return true;
       };
       if (ok) ok = issue_sdp(0);
@@ -501,55 +550,65 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
         ok = mbar_wait(&bars->ds_ready[t & 1], (uint32_t)(t >> 1) & 1, abort_word, p.status);
         if (!ok) break;
         tc_fence_after();
-        const int st = t % AB_STAGES;
-        const uint32_t sk = smem_u32(sKV + st * SM::kStage);
-        const uint32_t c_dp = tmem_base + (t & 1) * 128 + 64;
-#pragma unroll
-        for (int kk = 0; kk < AB_SUB / 16; ++kk) {
-          const uint32_t a_col = kk * 16;
-          umma_f16_ts(tmem_base + kColDQ, c_dp + a_col,
-                      umma_smem_desc_sw128(sk + kk * 2048, AB_SUB * 128, 1024), idesc_ts,
-                      (t > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(&bars->kv_empty[st]);
+        const int s3 = t % AB_ST3;
+        mma_grad<HD>(tmem_base + kColDQ, tmem_base + kColDP + (t & 1) * 128,
+                     sk + s3 * SM::kTile, t > 0);
+        umma_commit(&bars->k_empty[s3]);
       }
       if (ok) umma_commit(&bars->acc_done);
     }
   } else {
     const int quad = warp & 3;
-    const int part = (warp - 2) >> 2;  // quarter of the 64 columns this warp converts
+    const int part = (warp - 2) >> 2;  // quarter of the 128 columns this warp converts
     const int r = quad * 32 + lane;    // query row inside the block
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    const uint32_t t_s = tmem_base + lane_off + part * 32;
     const size_t lrow = ((size_t)b * p.Hq + h) * p.S + (size_t)i * AB_T + r;
     const float neg_lse2 = -p.lse[lrow] * kLog2e;
-    const float dl = p.delta[lrow];
+    const float neg_dl = -p.delta[lrow];
+    const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    const uint64_t nl2 = pack_f32x2(neg_lse2, neg_lse2);
+    const uint64_t nd2 = pack_f32x2(neg_dl, neg_dl);
     bool ok = true;
     for (int t = 0; t < nsteps; ++t) {
-      ok = mbar_wait(&bars->sdp_full[t & 1], (uint32_t)(t >> 1) & 1, abort_word, p.status);
+      ok = mbar_wait(&bars->s_full, (uint32_t)t & 1, abort_word, p.status);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t t_s = tmem_base + (t & 1) * 128 + lane_off + part * 16;
-      const uint32_t t_dp = t_s + 64;
-      // kv sub-blocks 2i and 2i+1 overlap the diagonal of query block i
-      const bool diag = t >= 2 * i;
-      const int k_rel = (t - 2 * i) * AB_SUB + part * 16;  // first key of this warp rel. to q row 0
-      uint32_t sv[16], dv[16];
-      tmem_ld_32x32b_x16(t_s, sv);
-      tmem_ld_32x32b_x16(t_dp, dv);
+      uint32_t sv[32];
+      tmem_ld_32x32b_x32(t_s, sv);
       tmem_ld_wait();
-      uint32_t ds[8];
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->s_free);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        float p0 = ex2_approx(fmaf(__uint_as_float(sv[2 * e]), p.scale_log2, neg_lse2));
-        float p1 = ex2_approx(fmaf(__uint_as_float(sv[2 * e + 1]), p.scale_log2, neg_lse2));
-        if (diag) {
-          if (k_rel + 2 * e > r) p0 = 0.f;
-          if (k_rel + 2 * e + 1 > r) p1 = 0.f;
-        }
-        ds[e] = pack_bf16x2(p0 * (__uint_as_float(dv[2 * e]) - dl),
-                            p1 * (__uint_as_float(dv[2 * e + 1]) - dl));
+      for (int e = 0; e < 16; ++e) {
+        const float2 x = unpack_f32x2(fma_f32x2(
+            pack_f32x2(__uint_as_float(sv[2 * e]), __uint_as_float(sv[2 * e + 1])), c2, nl2));
+        sv[2 * e] = __float_as_uint(ex2_approx(x.x));
+        sv[2 * e + 1] = __float_as_uint(ex2_approx(x.y));
       }
-      tmem_st_32x32b_x8(t_dp, ds);
+      if (t == i) {   // the diagonal block
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          if (part * 32 + e > r) sv[e] = 0u;
+      }
+      const uint32_t t_dp = t_s + kColDP + (t & 1) * 128;
+      ok = mbar_wait(&bars->dp_full[t & 1], (uint32_t)(t >> 1) & 1, abort_word, p.status);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t dv[32];
+      tmem_ld_32x32b_x32(t_dp, dv);
+      tmem_ld_wait();
+      uint32_t ds[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const float2 x = unpack_f32x2(mul_f32x2(
+            add_f32x2(pack_f32x2(__uint_as_float(dv[2 * e]), __uint_as_float(dv[2 * e + 1])),
+                      nd2),
+            pack_f32x2(__uint_as_float(sv[2 * e]), __uint_as_float(sv[2 * e + 1]))));
+        ds[e] = pack_bf16x2(x.x, x.y);
+      }
+      tmem_st_32x32b_x16(t_dp, ds);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -598,32 +657,27 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_bwd_dkv_kernel<HD>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         DkvSmem<HD>::kTotal);
+                                         AbSmem<HD>::kTotal);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(attn_bwd_dq_kernel<HD>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<HD>::kTotal);
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, AbSmem<HD>::kTotal);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
   const uint64_t T = (uint64_t)p.B * p.S;
-  // 128-row boxes for the resident tiles, 64-row boxes for the streamed ones
-  CUtensorMap tq, tk, tv, tdo, tq64, tk64, tv64, tdo64;
+  CUtensorMap tq, tk, tv, tdo;   // boxes of 64 columns x 128 rows
   int r = make_tmap_bf16_2d(&tq, q, (uint64_t)p.Hq * HD, T, ld_qkv, 64, AB_T);
   if (!r) r = make_tmap_bf16_2d(&tk, k, (uint64_t)p.Hkv * HD, T, ld_qkv, 64, AB_T);
   if (!r) r = make_tmap_bf16_2d(&tv, v, (uint64_t)p.Hkv * HD, T, ld_qkv, 64, AB_T);
   if (!r) r = make_tmap_bf16_2d(&tdo, dout, (uint64_t)p.Hq * HD, T, ld_do, 64, AB_T);
-  if (!r) r = make_tmap_bf16_2d(&tq64, q, (uint64_t)p.Hq * HD, T, ld_qkv, 64, AB_SUB);
-  if (!r) r = make_tmap_bf16_2d(&tk64, k, (uint64_t)p.Hkv * HD, T, ld_qkv, 64, AB_SUB);
-  if (!r) r = make_tmap_bf16_2d(&tv64, v, (uint64_t)p.Hkv * HD, T, ld_qkv, 64, AB_SUB);
-  if (!r) r = make_tmap_bf16_2d(&tdo64, dout, (uint64_t)p.Hq * HD, T, ld_do, 64, AB_SUB);
   if (r) return 1000 - r;
   const int n_blk = p.S / AB_T;
-  attn_bwd_dkv_kernel<HD><<<dim3(n_blk * p.Hkv * p.B), AB_THREADS, DkvSmem<HD>::kTotal, st>>>(
-      tq64, tk, tv, tdo64, p);
+  attn_bwd_dkv_kernel<HD><<<dim3(n_blk * p.Hkv * p.B), AB_THREADS, AbSmem<HD>::kTotal, st>>>(
+      tq, tk, tv, tdo, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  attn_bwd_dq_kernel<HD><<<dim3(n_blk, p.Hq, p.B), AB_THREADS, DqSmem<HD>::kTotal, st>>>(
-      tq, tk64, tv64, tdo, p);
+  attn_bwd_dq_kernel<HD><<<dim3(n_blk, p.Hq, p.B), AB_THREADS, AbSmem<HD>::kTotal, st>>>(
+      tq, tk, tv, tdo, p);
   return (int)cudaGetLastError();
 }
 
