@@ -55,31 +55,31 @@ int sm_count() {
   return n;
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA,
                      const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_cta_body<A_MN, B_MN>(&tmA, &tmB, p, blockIdx.x, gridDim.x, smem_raw);
+  gemm_cta_body<A_MN, B_MN, BN>(&tmA, &tmB, p, blockIdx.x, gridDim.x, smem_raw);
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int BN>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
                   cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, BN>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         GEMM_SMEM_BYTES);
+                                         GemmTile<BN>::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  gemm_bf16_kernel<A_MN, B_MN><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb, p);
+  gemm_bf16_kernel<A_MN, B_MN, BN><<<grid, GEMM_THREADS, GemmTile<BN>::kSmemBytes, st>>>(ta, tb, p);
   return (int)cudaGetLastError();
 }
 
-int make_gemm_tmaps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B, int M, int N,
-                    int K, int lda, int ldb, int a_mn, int b_mn) {
+static int make_gemm_tmaps_bn(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B,
+                              int M, int N, int K, int lda, int ldb, int a_mn, int b_mn, int bn) {
   int r;
   if (a_mn)
     r = make_tmap_bf16_2d(ta, A, M, K, lda, 64, 64);
@@ -89,16 +89,253 @@ int make_gemm_tmaps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void*
   if (b_mn)
     r = make_tmap_bf16_2d(tb, B, N, K, ldb, 64, 64);
   else
-    r = make_tmap_bf16_2d(tb, B, K, N, ldb, 64, GEMM_BN);
+    r = make_tmap_bf16_2d(tb, B, K, N, ldb, 64, bn);
   return r;
 }
+int make_gemm_tmaps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B, int M, int N,
+                    int K, int lda, int ldb, int a_mn, int b_mn) {
+  return make_gemm_tmaps_bn(ta, tb, A, B, M, N, K, lda, ldb, a_mn, b_mn, GEMM_BN);
+}
 
+template <int BN>
+static int launch_gemm_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                          int a_mn, int b_mn, int grid, cudaStream_t st) {
+  if (a_mn && b_mn) return launch<true, true, BN>(ta, tb, p, grid, st);
+  if (a_mn) return launch<true, false, BN>(ta, tb, p, grid, st);
+  if (b_mn) return launch<false, true, BN>(ta, tb, p, grid, st);
+  return launch<false, false, BN>(ta, tb, p, grid, st);
+}
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int a_mn,
                 int b_mn, int grid, cudaStream_t st) {
-  if (a_mn && b_mn) return launch<true, true>(ta, tb, p, grid, st);
-  if (a_mn) return launch<true, false>(ta, tb, p, grid, st);
-  if (b_mn) return launch<false, true>(ta, tb, p, grid, st);
-  return launch<false, false>(ta, tb, p, grid, st);
+  return launch_gemm_bn<GEMM_BN>(ta, tb, p, a_mn, b_mn, grid, st);
+}
+
+// ------------------------------------------------------------------- split over K
+// A product with fewer tiles than SMs is bound by what one SM can fetch (64 to 76 B/clk by
+// TMA, measured), not by the tensor cores.  Here a cluster of SPLIT CTAs shares one 128 x BN
+// tile: each multiplies its part of K, leaves the fp32 partial tile in its own shared memory
+// (the stage buffers are free by then), and after a cluster barrier each CTA adds up
+// 128 / SPLIT rows of all parts over distributed shared memory, in rank order, and stores
+// them.  No workspace, no second launch, the same bits on every run.
+// 64x4096x14336: 69.8 us as 256x256 pair tiles -> 25.7 us (4.5 TB/s); 64x4096x4096: 24.3 -> 10.1 us.
+template <int BN, int SPLIT>
+struct SplitTile {
+  static constexpr int kLd = BN + 4;   // floats per row of the partial tile: no bank conflicts
+  static_assert(GEMM_BM * kLd * 4 <= GemmTile<BN>::kStages * GemmTile<BN>::kStageBytes, "");
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(cluster_addr)
+               : "memory");
+  return v;
+}
+
+template <bool A_MN, bool B_MN, int BN, int SPLIT>
+__global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+    gemm_split_kernel(const __grid_constant__ CUtensorMap tmA,
+                      const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+  constexpr int STAGES = GemmTile<BN>::kStages;
+  constexpr int STAGE_BYTES = GemmTile<BN>::kStageBytes;
+  constexpr int LD = SplitTile<BN, SPLIT>::kLd;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  auto* sh = reinterpret_cast<GemmShared<STAGES>*>(smem + STAGES * STAGE_BYTES);
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int part = (int)cluster_ctarank();
+  const int tile = (int)blockIdx.x / SPLIT;
+  const int m_blocks = (p.M + GEMM_BM - 1) / GEMM_BM;
+  const int m0 = (tile % m_blocks) * GEMM_BM, n0 = (tile / m_blocks) * BN;
+  const int all_iters = (p.K + GEMM_BK - 1) / GEMM_BK;   // >= SPLIT (launcher)
+  const int k_begin = (int)((long long)all_iters * part / SPLIT);
+  const int k_end = (int)((long long)all_iters * (part + 1) / SPLIT);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&sh->full[s], 1);
+      mbar_init(&sh->empty[s], 1);
+    }
+    mbar_init(&sh->tmem_full[0], 1);
+    sh->abort_word = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&sh->tmem_base, BN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = sh->tmem_base;
+  volatile int* abort_word = &sh->abort_word;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int k = k_begin; k < k_end; ++k) {
+        if (!mbar_wait(&sh->empty[stage], phase ^ 1, abort_word, p.status)) break;
+        uint8_t* sa = smem + stage * STAGE_BYTES;
+        uint8_t* sb = sa + GEMM_A_BYTES;
+        mbar_expect_tx(&sh->full[stage], STAGE_BYTES);
+        const int k0 = k * GEMM_BK;
+        if (A_MN) {
+#pragma unroll
+          for (int j = 0; j < GEMM_BM / 64; ++j)
+            tma_load_2d(sa + j * 8192, &tmA, &sh->full[stage], m0 + j * 64, k0);
+        } else {
+          tma_load_2d(sa, &tmA, &sh->full[stage], k0, m0);
+        }
+        if (B_MN) {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j)
+            tma_load_2d(sb + j * 8192, &tmB, &sh->full[stage], n0 + j * 64, k0);
+        } else {
+          tma_load_2d(sb, &tmB, &sh->full[stage], k0, n0);
+        }
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int k = k_begin; k < k_end; ++k) {
+        ok = mbar_wait(&sh->full[stage], phase, abort_word, p.status);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
+        const uint32_t sb = sa + GEMM_A_BYTES;
+#pragma unroll
+        for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
+          const uint64_t da = A_MN ? umma_smem_desc_sw128(sa + kk * 2048, 8192, 1024)
+                                   : umma_smem_desc_sw128(sa + kk * 32, 16, 1024);
+          const uint64_t db = B_MN ? umma_smem_desc_sw128(sb + kk * 2048, 8192, 1024)
+                                   : umma_smem_desc_sw128(sb + kk * 32, 16, 1024);
+          umma_f16(tmem_base, da, db, idesc, (k > k_begin || kk > 0) ? 1u : 0u);
+        }
+        umma_commit(&sh->empty[stage]);
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+      if (ok) umma_commit(&sh->tmem_full[0]);
+    }
+  } else {
+    // every load of this CTA has landed and every MMA has read its stage once tmem_full is
+    // signalled, so the stage buffers can take the partial tile
+    const int quad = warp & 3;
+    if (mbar_wait(&sh->tmem_full[0], 0, abort_word, p.status)) {
+      tc_fence_after();
+      float* row = reinterpret_cast<float*>(smem) + (quad * 32 + lane) * LD;
+#pragma unroll 1
+      for (int c = 0; c < BN / 32; ++c) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(tmem_base + c * 32 + ((uint32_t)(quad * 32) << 16), v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<uint4*>(row + c * 32 + q * 4) =
+              make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+      }
+    }
+  }
+  tc_fence_before();
+  cluster_sync_all();   // all parts are in shared memory
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, BN);
+  }
+  {
+    constexpr int ROWS = GEMM_BM / SPLIT;
+    const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
+                        (!p.R || (((p.ldr & 7) == 0) &&
+                                  ((reinterpret_cast<uintptr_t>(p.R) & 15) == 0)));
+    const uint32_t base = smem_u32(smem);
+    for (int it = threadIdx.x; it < ROWS * (BN / 8); it += GEMM_THREADS) {
+      const int r = part * ROWS + it / (BN / 8), c = (it % (BN / 8)) * 8;
+      const int row = m0 + r, col = n0 + c;
+      if (row >= p.M || col >= p.N) continue;
+      float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < SPLIT; ++s) {
+        const uint32_t src = mapa_u32(base + (uint32_t)(r * LD + c) * 4, s);
+        const float4 x = ld_cluster_f4(src), y = ld_cluster_f4(src + 16);
+        f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w;
+        f[4] += y.x; f[5] += y.y; f[6] += y.z; f[7] += y.w;
+      }
+      gemm_store8(p, f, row, col, vec_ok);
+    }
+  }
+  cluster_sync_all();   // keep the parts until every CTA of the cluster has read them
+}
+
+// Number of clusters of SPLIT CTAs that can be resident at once; 0 when there is no answer.
+template <bool A_MN, bool B_MN, int BN, int SPLIT>
+static int split_capacity() {
+  static int cap = -1;
+  if (cap >= 0) return cap;
+  if (cudaFuncSetAttribute(gemm_split_kernel<A_MN, B_MN, BN, SPLIT>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           GemmTile<BN>::kSmemBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(SPLIT * (sm_count() / SPLIT));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = GemmTile<BN>::kSmemBytes;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = SPLIT;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<A_MN, B_MN, BN, SPLIT>, &cfg) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  cap = n;
+  return cap;
+}
+
+template <bool A_MN, bool B_MN, int BN, int SPLIT>
+static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                        int tiles, cudaStream_t st) {
+  if (split_capacity<A_MN, B_MN, BN, SPLIT>() <= 0) return 1002;
+  gemm_split_kernel<A_MN, B_MN, BN, SPLIT>
+      <<<tiles * SPLIT, GEMM_THREADS, GemmTile<BN>::kSmemBytes, st>>>(ta, tb, p);
+  return (int)cudaGetLastError();
+}
+template <int BN, int SPLIT>
+static int launch_split_ab(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                           int a_mn, int b_mn, int tiles, cudaStream_t st) {
+  if (a_mn && b_mn) return launch_split<true, true, BN, SPLIT>(ta, tb, p, tiles, st);
+  if (a_mn) return launch_split<true, false, BN, SPLIT>(ta, tb, p, tiles, st);
+  if (b_mn) return launch_split<false, true, BN, SPLIT>(ta, tb, p, tiles, st);
+  return launch_split<false, false, BN, SPLIT>(ta, tb, p, tiles, st);
+}
+template <int BN>
+static int launch_split_n(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                          int a_mn, int b_mn, int split, int tiles, cudaStream_t st) {
+  if (split == 8) return launch_split_ab<BN, 8>(ta, tb, p, a_mn, b_mn, tiles, st);
+  if (split == 4) return launch_split_ab<BN, 4>(ta, tb, p, a_mn, b_mn, tiles, st);
+  return launch_split_ab<BN, 2>(ta, tb, p, a_mn, b_mn, tiles, st);
 }
 
 // ------------------------------------------------------------------ CTA-pair variant
@@ -176,8 +413,49 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams&
   return launch2<false, false>(ta, tb, p, st);
 }
 
-// 1: single-CTA 128x256 tiles; 2: CTA-pair 256x256 tiles.
+// 1: single-CTA 128x256 tiles; 2: CTA-pair 256x256 tiles, or smaller ones where gemm_plan
+// finds them faster.
 static int g_gemm_impl = 2;
+
+// Tile and K split of the plain product under implementation 2: the smallest estimate of
+//   t0 + waves * (64-deep steps of one CTA or pair) * c
+// with the microseconds measured on this chip.  c is what limits a step: 32 KB per SM and the
+// tensor pipe for the pair, the 24 to 48 KB that one SM fetches for the others.  t0 is launch,
+// first load, last epilogue; a split adds its cluster barriers and the exchange.  Estimate ->
+// measured, us: 8192x1024x1024 pair 18.0 -> 18.1; 2048x4096x4096 pair 51.2 -> 50.2, 128x256
+// 54.5 -> 55.1, 128x128 67.0 -> 68.7; 2048^3 128x256 17.5 -> 16.9, pair 18.0 -> 18.6;
+// 1000x2048x3072 128x128 16.1 -> 15.0, pair 23.6 -> 20.5; 200x768x256 128x64 4.4 -> 4.7, pair
+// 8.4 -> 9.0; 64x4096x4096 128x128 in 4 parts 10.3 -> 10.1, 128x64 in 2 parts 10.8 -> 11.1.
+struct GemmPlan {
+  int bn;      // 0: the CTA pair's 256x256 tile, else the columns of a single CTA's 128-row tile
+  int split;   // CTAs of a cluster that share a tile along K
+};
+static GemmPlan gemm_plan(int M, int N, int K) {
+  const int iters = (K + GEMM_BK - 1) / GEMM_BK;
+  const auto div = [](long long a, long long b) { return (a + b - 1) / b; };
+  const int sms = sm_count();
+  GemmPlan best = {0, 1};
+  float t = 7.0f + 0.345f * iters * div(div(M, G2_BM) * div(N, G2_BN), sms / 2);
+  struct { int bn; float t0, c, t_split[3]; } const kinds[] = {
+      {256, 5.2f, 0.385f, {0.f, 0.f, 0.f}},
+      {128, 4.3f, 0.245f, {1.05f, 2.1f, 3.2f}},   // splits of 2, 4, 8
+      {64, 3.6f, 0.200f, {0.8f, 1.5f, 2.3f}},
+  };
+  for (const auto& k : kinds) {
+    const long long tiles = div(M, GEMM_BM) * div(N, k.bn);
+    const float u = k.t0 + k.c * iters * div(tiles, sms);
+    if (u < t) t = u, best = {k.bn, 1};
+    if (k.bn == 256) continue;
+    for (int i = 0; i < 3; ++i) {
+      const int split = 2 << i;
+      // one wave only: clusters of 8 fill 16 of every GPC's 18 to 20 SMs
+      if (tiles * split > (split == 2 ? sms - 4 : sms * 7 / 8) || iters < 2 * split) break;
+      const float v = k.t0 + k.t_split[i] + k.c * div(iters, split);
+      if (v < t) t = v, best = {k.bn, split};
+    }
+  }
+  return best;
+}
 
 }  // namespace mb200
 
@@ -187,9 +465,6 @@ extern "C" int mb200_gemm_bf16(const void* A, const void* B, void* C, const void
                                int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn,
                                int accumulate, int* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  CUtensorMap ta, tb;
-  int r = make_gemm_tmaps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
-  if (r) return 1000 - r;
   GemmParams p{};
   p.C = reinterpret_cast<__nv_bfloat16*>(C);
   p.R = reinterpret_cast<const __nv_bfloat16*>(R);
@@ -204,15 +479,22 @@ extern "C" int mb200_gemm_bf16(const void* A, const void* B, void* C, const void
   p.ldb = ldb;
   p.n_blk_rot = 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (g_gemm_impl == 2) {
-    CUtensorMap ta2, tb2;
-    r = make_gemm2_tmaps(&ta2, &tb2, A, B, M, N, K, lda, ldb, a_mn, b_mn);
-    if (r) return 1000 - r;
-    return launch_gemm2(ta2, tb2, p, a_mn, b_mn, st);
+  CUtensorMap ta, tb;
+  const GemmPlan plan = g_gemm_impl == 2 ? gemm_plan(M, N, K) : GemmPlan{GEMM_BN, 1};
+  const int bn = plan.bn;
+  if (bn == 0) {
+    const int r = make_gemm2_tmaps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
+    return r ? 1000 - r : launch_gemm2(ta, tb, p, a_mn, b_mn, st);
   }
-  const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + GEMM_BN - 1) / GEMM_BN);
-  int grid = sm_count();
-  if (tiles < grid) grid = tiles;
+  const int r = make_gemm_tmaps_bn(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn, bn);
+  if (r) return 1000 - r;
+  const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + bn - 1) / bn);
+  if (plan.split > 1)
+    return bn == 64 ? launch_split_n<64>(ta, tb, p, a_mn, b_mn, plan.split, tiles, st)
+                    : launch_split_n<128>(ta, tb, p, a_mn, b_mn, plan.split, tiles, st);
+  const int grid = tiles < sm_count() ? tiles : sm_count();
+  if (bn == 64) return launch_gemm_bn<64>(ta, tb, p, a_mn, b_mn, grid, st);
+  if (bn == 128) return launch_gemm_bn<128>(ta, tb, p, a_mn, b_mn, grid, st);
   return launch_gemm(ta, tb, p, a_mn, b_mn, grid, st);
 }
 

@@ -112,7 +112,7 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(tmA);
       tma_prefetch_desc(tmB);
       const uint32_t full0 = mapa_u32(smem_u32(&sh->full[0]), 0);  // even CTA's barriers
@@ -176,7 +176,7 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
     }
   } else if (warp == 1) {
     // ------------------------------------------------- MMA issuer (even CTA only)
-    if (cta == 0 && lane == 0) {
+    if (cta == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(G2_BM, G2_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;

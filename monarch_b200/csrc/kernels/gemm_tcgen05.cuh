@@ -21,12 +21,17 @@ namespace mb200 {
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BN = 256;
 constexpr int GEMM_BK = 64;
-constexpr int GEMM_STAGES = 4;
 constexpr int GEMM_THREADS = 192;  // warp0: TMA, warp1: MMA, warps 2-5: epilogue
 constexpr int GEMM_A_BYTES = GEMM_BM * GEMM_BK * 2;
-constexpr int GEMM_B_BYTES = GEMM_BN * GEMM_BK * 2;
-constexpr int GEMM_STAGE_BYTES = GEMM_A_BYTES + GEMM_B_BYTES;
-constexpr int GEMM_SMEM_BYTES = GEMM_STAGES * GEMM_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+// The tile is 128 x BN: 256 columns, or 128 or 64 for products with few tiles.  192 KB of
+// stages in every case.
+template <int BN>
+struct GemmTile {
+  static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 6 : 8;
+  static constexpr int kStageBytes = GEMM_A_BYTES + BN * GEMM_BK * 2;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+};
+constexpr int GEMM_SMEM_BYTES = GemmTile<GEMM_BN>::kSmemBytes;
 
 struct GemmParams {
   __nv_bfloat16* C;
@@ -92,6 +97,46 @@ __device__ __forceinline__ int gemm_dyn_k(const GemmParams& p) {
   if (!p.dyn_k) return p.K;
   const int k = *reinterpret_cast<const volatile int*>(p.dyn_k);
   return k < p.K ? k : p.K;
+}
+
+// Eight finished columns of one output row (+ residual, + C).  vec_ok: C and R and their
+// leading dimensions are 16-byte aligned.
+__device__ __forceinline__ void gemm_store8(const GemmParams& p, float (&f)[8], int row, int col,
+                                            bool vec_ok) {
+  __nv_bfloat16* cp = p.C + (size_t)row * p.ldc + col;
+  const __nv_bfloat16* rp = p.R ? p.R + (size_t)row * p.ldr + col : nullptr;
+  if (vec_ok && col + 8 <= p.N) {
+    if (rp) {
+      const uint4 r4 = *reinterpret_cast<const uint4*>(rp);
+      const float2 a = unpack_bf16x2(r4.x), b = unpack_bf16x2(r4.y), c = unpack_bf16x2(r4.z),
+                   d = unpack_bf16x2(r4.w);
+      f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y;
+      f[4] += c.x; f[5] += c.y; f[6] += d.x; f[7] += d.y;
+    }
+    if (p.accumulate) {
+      const uint4 r4 = *reinterpret_cast<const uint4*>(cp);
+      const float2 a = unpack_bf16x2(r4.x), b = unpack_bf16x2(r4.y), c = unpack_bf16x2(r4.z),
+                   d = unpack_bf16x2(r4.w);
+      f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y;
+      f[4] += c.x; f[5] += c.y; f[6] += d.x; f[7] += d.y;
+    }
+    uint4 o;
+    o.x = pack_bf16x2(f[0], f[1]);
+    o.y = pack_bf16x2(f[2], f[3]);
+    o.z = pack_bf16x2(f[4], f[5]);
+    o.w = pack_bf16x2(f[6], f[7]);
+    *reinterpret_cast<uint4*>(cp) = o;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (col + i < p.N) {
+        float x = f[i];
+        if (rp) x += __bfloat162float(rp[i]);
+        if (p.accumulate) x += __bfloat162float(cp[i]);
+        cp[i] = __float2bfloat16(x);
+      }
+    }
+  }
 }
 
 // Shared by both bodies: write one 32-column strip of an accumulator row.
@@ -190,35 +235,38 @@ __device__ __forceinline__ bool gemm_wait_rows(const uint32_t* ready, uint32_t t
   return ok;
 }
 
+template <int STAGES>
 struct GemmShared {
-  uint64_t full[GEMM_STAGES];
-  uint64_t empty[GEMM_STAGES];
+  uint64_t full[STAGES];
+  uint64_t empty[STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   volatile int abort_word;
 };
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int BN = GEMM_BN>
 __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUtensorMap* tmB,
                                               const GemmParams& p, int vcta, int nvcta,
                                               uint8_t* smem_raw) {
+  constexpr int STAGES = GemmTile<BN>::kStages;
+  constexpr int STAGE_BYTES = GemmTile<BN>::kStageBytes;
   // 1024-byte aligned stage buffers (required by the 128-byte swizzle atoms).
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  GemmShared* sh = reinterpret_cast<GemmShared*>(smem + GEMM_STAGES * GEMM_STAGE_BYTES);
+  auto* sh = reinterpret_cast<GemmShared<STAGES>*>(smem + STAGES * STAGE_BYTES);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int M = gemm_dyn_m(p);
   const int Kd = gemm_dyn_k(p);
   const int m_blocks = (M + GEMM_BM - 1) / GEMM_BM;
-  const int n_blocks = (p.N + GEMM_BN - 1) / GEMM_BN;
+  const int n_blocks = (p.N + BN - 1) / BN;
   const int k_iters = (Kd + GEMM_BK - 1) / GEMM_BK;
   const int num_tiles = m_blocks * n_blocks;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < GEMM_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sh->full[s], 1);
       mbar_init(&sh->empty[s], 1);
     }
@@ -230,7 +278,7 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(&sh->tmem_base, 512);
+    tmem_alloc(&sh->tmem_base, 2 * BN);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -241,7 +289,7 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(tmA);
       tma_prefetch_desc(tmB);
       int stage = 0;
@@ -250,11 +298,11 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
         const int m_blk = t % m_blocks;
         int n_blk = t / m_blocks + p.n_blk_rot;
         if (n_blk >= n_blocks) n_blk -= n_blocks;
-        const int m0 = m_blk * GEMM_BM, n0 = n_blk * GEMM_BN;
+        const int m0 = m_blk * GEMM_BM, n0 = n_blk * BN;
         bool ok = true;
         if (p.b_ready) {
           // both ends of the block: a 256-row block may straddle several flag ranges
-          int last_row = n0 + GEMM_BN - 1;
+          int last_row = n0 + BN - 1;
           if (last_row >= p.N) last_row = p.N - 1;
           ok = gemm_wait_rows(p.b_ready, p.b_ready_target, p.flag_chunk_elems, p.b_flag_elem0,
                               p.ldb, n0, last_row, p.K, p.status);
@@ -275,9 +323,9 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
             failed = true;
             break;
           }
-          uint8_t* sa = smem + stage * GEMM_STAGE_BYTES;
+          uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + GEMM_A_BYTES;
-          mbar_expect_tx(&sh->full[stage], GEMM_STAGE_BYTES);
+          mbar_expect_tx(&sh->full[stage], STAGE_BYTES);
           const int k0 = k * GEMM_BK;
           if (A_MN) {
 #pragma unroll
@@ -288,12 +336,12 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
           }
           if (B_MN) {
 #pragma unroll
-            for (int j = 0; j < GEMM_BN / 64; ++j)
+            for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(sb + j * 8192, tmB, &sh->full[stage], n0 + j * 64, k0);
           } else {
             tma_load_2d(sb, tmB, &sh->full[stage], k0, n0);
           }
-          if (++stage == GEMM_STAGES) {
+          if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
@@ -303,8 +351,8 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, GEMM_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -312,7 +360,7 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
       for (int t = vcta; t < num_tiles; t += nvcta) {
         if (!mbar_wait(&sh->tmem_empty[acc], acc_phase ^ 1, abort_word, p.status)) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * GEMM_BN;
+        const uint32_t d_tmem = tmem_base + acc * BN;
         bool failed = false;
         for (int k = 0; k < k_iters; ++k) {
           if (!mbar_wait(&sh->full[stage], phase, abort_word, p.status)) {
@@ -320,7 +368,7 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * GEMM_STAGE_BYTES);
+          const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t sb = sa + GEMM_A_BYTES;
 #pragma unroll
           for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
@@ -331,7 +379,7 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
             umma_f16(d_tmem, da, db, idesc, (k > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&sh->empty[stage]);  // stage reusable once these MMAs retire
-          if (++stage == GEMM_STAGES) {
+          if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
@@ -357,12 +405,12 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
       int n_blk = t / m_blocks + p.n_blk_rot;
       if (n_blk >= n_blocks) n_blk -= n_blocks;
       const int row = m_blk * GEMM_BM + quad * 32 + lane;
-      const int n0 = n_blk * GEMM_BN;
+      const int n0 = n_blk * BN;
       if (!mbar_wait(&sh->tmem_full[acc], acc_phase, abort_word, p.status)) break;
       tc_fence_after();
-      const uint32_t t_base = tmem_base + acc * GEMM_BN + ((uint32_t)(quad * 32) << 16);
+      const uint32_t t_base = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < GEMM_BN / 32; ++c) {
+      for (int c = 0; c < BN / 32; ++c) {
         uint32_t v[32];
         tmem_ld_32x32b_x32(t_base + c * 32, v);
         tmem_ld_wait();
@@ -387,7 +435,7 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, 2 * BN);
   }
 }
 

@@ -158,7 +158,8 @@ def bounds_register(ptr: int, nbytes: int, device=None) -> None:
 
 def set_gemm_impl(impl: int) -> None:
     """Select the GEMM kernel behind :func:`monarch_b200.ops.gemm`: 1 = single-CTA
-    128x256 tiles, 2 = CTA-pair (``cta_group::2``) 256x256 tiles."""
+    128x256 tiles, 2 = CTA-pair (``cta_group::2``) 256x256 tiles, or smaller single-CTA ones
+    (split along K by a cluster where that helps) for products with few tiles."""
     rc = lib().mb200_gemm_set_impl(int(impl))
     if rc:
         raise KernelError(f"unknown GEMM implementation {impl}")

@@ -220,3 +220,30 @@ def test_optimizer_overlapped_with_backward_is_bit_identical():
         assert torch.equal(a_st.params, b_st.params) and torch.equal(a_st.master, b_st.master)
         assert torch.equal(a_st.m, b_st.m) and torch.equal(a_st.v, b_st.v)
         assert a_st.step_count == b_st.step_count == 2
+
+
+# (M, N, K): what each tile of the plain product covers -- 128x64 and its splits (few rows, long
+# K; fewer rows and columns than a tile; remainders in M, N and K), 128x128 and its splits,
+# 128x256, and one row
+@pytest.mark.parametrize("M,N,K_", [(200, 768, 256), (1, 264, 4096), (64, 512, 4104), (96, 4096, 4096),
+                                    (8, 24, 1032), (333, 1496, 1096), (1000, 2048, 1544),
+                                    (257, 6144, 1024), (2048, 2048, 2056)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+def test_gemm_tile_choice(M, N, K_, a_mn, b_mn):
+    """Every tile and split the product can choose, against 64 bits: the only rounding is that
+    of the bf16 result (2^-9 at most, 1.7e-3 in the 2-norm) plus fp32 sums of K terms."""
+    if a_mn and M % 8:
+        M += 8 - M % 8
+    torch.manual_seed(4)
+    a = torch.randn((K_, M) if a_mn else (M, K_), device="cuda", dtype=bf16)
+    b = torch.randn((K_, N) if b_mn else (N, K_), device="cuda", dtype=bf16)
+    r = torch.randn(M, N, device="cuda", dtype=bf16)
+    wide = torch.full((M, N + 8), 7.0, device="cuda", dtype=bf16)
+    ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=wide[:, :N], residual=r)
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double() + r.double()
+    err = ((wide[:, :N].double() - ref).norm() / ref.norm()).item()
+    assert err < 2.5e-3, err
+    assert (wide[:, N:] == 7).all()
+    first = wide[:, :N].clone()
+    ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=wide[:, :N], accumulate=True)
+    assert _rel(wide[:, :N], ref - r.double() + first.double()) < 2.5e-3
