@@ -99,6 +99,8 @@ class ParamSpec:
     name: str
     shape: tuple
     offset: int  # element offset inside its unit
+    numel: int = 0
+    strides: tuple = ()   # of a contiguous tensor of this shape
 
 
 @dataclass
@@ -136,10 +138,11 @@ class ParamLayout:
             u = Unit(name, off, 0, seed_id=seed_id)
             o = 0
             for n, shape in specs:
-                u.params.append(ParamSpec(n, tuple(shape), o))
-                numel = 1
-                for s in shape:
+                numel, strides = 1, []
+                for s in reversed(shape):
+                    strides.insert(0, numel)
                     numel *= s
+                u.params.append(ParamSpec(n, tuple(shape), o, numel, tuple(strides)))
                 o += _round_up(numel, 8)
             u.size = _round_up(o, self.ALIGN)
             off += u.size
@@ -173,13 +176,13 @@ class ParamLayout:
         raise KeyError(name)
 
     def views(self, unit: Unit, flat_unit: torch.Tensor) -> dict:
-        out = {}
-        for p in unit.params:
-            n = 1
-            for s in p.shape:
-                n *= s
-            out[p.name] = flat_unit[p.offset: p.offset + n].view(p.shape)
-        return out
+        if flat_unit.stride() != (1,) or flat_unit.shape[0] < unit.size:
+            return {p.name: flat_unit[p.offset: p.offset + p.numel].view(p.shape)
+                    for p in unit.params}
+        # one call per parameter instead of a slice and a view
+        base = flat_unit.storage_offset()
+        return {p.name: flat_unit.as_strided(p.shape, p.strides, base + p.offset)
+                for p in unit.params}
 
 
 class LocalParamStore:

@@ -20,11 +20,14 @@ def _p(t):
     return 0 if t is None else t.data_ptr()
 
 
-def _rowmajor(t: torch.Tensor) -> torch.Tensor:
+def _rowmajor(t: torch.Tensor):
+    """(t with unit inner stride, its leading dimension)."""
     assert t.dim() == 2
-    if t.stride(1) != 1 or t.stride(0) < t.shape[1]:
+    ld, inner = t.stride()
+    if inner != 1 or ld < t.shape[1]:
         t = t.contiguous()
-    return t
+        ld = t.stride(0)
+    return t, ld
 
 
 def gemm(a, b, *, a_mn=False, b_mn=False, out=None, residual=None, accumulate=False):
@@ -34,25 +37,34 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, residual=None, accumulate=Fa
     (``b_mn=False``, i.e. out = a @ b.T) or [K,N] (``b_mn=True``).  bf16 in, fp32
     accumulation on the tensor cores (tcgen05, accumulator in TMEM), bf16 out.
     """
-    a = _rowmajor(a)
-    b = _rowmajor(b)
-    M, Ka = (a.shape[1], a.shape[0]) if a_mn else a.shape
-    N, Kb = (b.shape[1], b.shape[0]) if b_mn else b.shape
+    a, lda = _rowmajor(a)
+    b, ldb = _rowmajor(b)
+    M, Ka = a.shape
+    if a_mn:
+        M, Ka = Ka, M
+    N, Kb = b.shape
+    if b_mn:
+        N, Kb = Kb, N
     assert Ka == Kb, (a.shape, b.shape, a_mn, b_mn)
     if out is None:
         assert not accumulate
         out = torch.empty(M, N, dtype=a.dtype, device=a.device)
-    assert out.shape == (M, N) and out.stride(1) == 1
+        ldc = N
+    else:
+        ldc, inner = out.stride()
+        assert out.shape == (M, N) and inner == 1
     if not a.is_cuda:
         out.copy_(R.gemm(a, b, a_mn, b_mn, residual, out if accumulate else None).to(out.dtype))
         return out
     assert a.dtype == bf16 and b.dtype == bf16 and out.dtype == bf16
+    res, ldr = 0, 0
     if residual is not None:
-        assert residual.shape == (M, N) and residual.stride(1) == 1 and residual.dtype == bf16
+        ldr, inner = residual.stride()
+        assert residual.shape == (M, N) and inner == 1 and residual.dtype == bf16
+        res = residual.data_ptr()
     rc = K.lib().mb200_gemm_bf16(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), _p(residual), M, N, Ka, a.stride(0),
-        b.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
-        int(a_mn), int(b_mn), int(accumulate), K.status_word(a.device).data_ptr(), K.stream_ptr())
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), res, M, N, Ka, lda, ldb, ldc, ldr,
+        int(a_mn), int(b_mn), int(accumulate), K.status_ptr(a), K.stream_ptr())
     K.check(rc, "gemm_bf16")
     return out
 
@@ -209,8 +221,12 @@ def sumsq(x, out=None):
 def have_attention_kernel() -> bool:
     """True when the tcgen05 flash-attention kernels (forward and backward) are in the
     loaded library and not disabled with ``MB200_ATTN=sdpa``."""
-    if not torch.cuda.is_available() or os.environ.get("MB200_ATTN", "") == "sdpa":
+    if os.environ.get("MB200_ATTN", "") == "sdpa" or not torch.cuda.is_available():
         return False
+    return _lib_has_attention()
+
+
+def _lib_has_attention() -> bool:
     l = K.lib()
     return hasattr(l, "mb200_attn_fwd") and hasattr(l, "mb200_attn_bwd")
 
@@ -232,7 +248,7 @@ def attention_fwd(qkv, B, S, Hq, Hkv, hd, scale=None, need_bwd=True):
     ctx.qkv, ctx.B, ctx.S, ctx.Hq, ctx.Hkv, ctx.hd, ctx.scale = qkv, B, S, Hq, Hkv, hd, scale
     ctx.graph = None
     T = B * S
-    if qkv.is_cuda and have_attention_kernel():
+    if qkv.is_cuda and os.environ.get("MB200_ATTN", "") != "sdpa" and _lib_has_attention():
         o = torch.empty(T, Hq * hd, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(B, Hq, S, dtype=torch.float32, device=qkv.device)
         q = qkv
@@ -240,7 +256,7 @@ def attention_fwd(qkv, B, S, Hq, Hkv, hd, scale=None, need_bwd=True):
         v = qkv[:, (Hq + Hkv) * hd:]
         K.check(K.lib().mb200_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                                        lse.data_ptr(), B, S, Hq, Hkv, hd, qkv.stride(0),
-                                       o.stride(0), scale, K.status_word(qkv.device).data_ptr(),
+                                       o.stride(0), scale, K.status_ptr(qkv),
                                        K.stream_ptr()), "attn_fwd")
         ctx.o, ctx.lse = o, lse
         return o, ctx
@@ -287,7 +303,7 @@ def attention_bwd(ctx: AttnCtx, do):
                                        delta.data_ptr(), dqkv.data_ptr(), dk.data_ptr(),
                                        dv.data_ptr(), B, S, Hq, Hkv, hd, qkv.stride(0),
                                        ctx.o.stride(0), dqkv.stride(0), ctx.scale,
-                                       K.status_word(qkv.device).data_ptr(), K.stream_ptr()),
+                                       K.status_ptr(qkv), K.stream_ptr()),
                 "attn_bwd", 3)
         return dqkv
     q, k, v, o2 = ctx.graph

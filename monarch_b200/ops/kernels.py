@@ -182,6 +182,12 @@ def status_word(device: torch.device | int | None = None) -> torch.Tensor:
     return t
 
 
+def status_ptr(t: torch.Tensor) -> int:
+    """Address of the status word of the device that holds ``t``."""
+    w = _status.get(t.get_device())
+    return (status_word(t.device) if w is None else w).data_ptr()
+
+
 _STATUS_TEXT = {1: "mbarrier wait timed out inside a kernel",
                 2: "wait on a peer/ready flag timed out inside a kernel",
                 3: "kernel rejected its arguments",
@@ -235,7 +241,9 @@ class StatusWatch:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream: 0.1 us, where building a
+    ``torch.cuda.Stream`` object for it takes 3.4 us, a quarter of a small operator's call."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def check(rc: int, what: str, n_launch: int = 1) -> None:
