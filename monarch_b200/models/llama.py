@@ -389,18 +389,19 @@ class LlamaEngine:
         x2 = ops.gemm(attn, w["wo"], residual=x)
         return x2, (x, rstd1, h1, actx, attn)
 
-    def _mlp_fwd(self, w: dict, x2: torch.Tensor, keep: bool):
-        """x2 -> x2 + mlp(norm(x2))."""
+    def _mlp_fwd(self, w: dict, x2: torch.Tensor, keep: bool, need_out: bool = True):
+        """x2 -> x2 + mlp(norm(x2)); without ``need_out`` only what the backward reads (the
+        down projection's result is no part of it) and None in its place."""
         h2, rstd2 = ops.rmsnorm_fwd(x2, w["mlp_norm"], self.cfg.eps)
         gu = _unit_gemm(w, h2, "w_gu")
         hmid = ops.swiglu_fwd(gu)
-        y = ops.gemm(hmid, w["w_down"], residual=x2)
+        y = ops.gemm(hmid, w["w_down"], residual=x2) if need_out else None
         return y, ((x2, rstd2, h2, gu, hmid) if keep else None)
 
     def _layer_fwd(self, w: dict, x: torch.Tensor, B: int, S: int, keep: bool,
-                   attn_saved=None):
+                   attn_saved=None, need_out: bool = True):
         x2, sa = self._attn_fwd(w, x, B, S, keep, attn_saved)
-        y, sm = self._mlp_fwd(w, x2, keep)
+        y, sm = self._mlp_fwd(w, x2, keep, need_out)
         if keep:
             return y, (sa, sm)
         actx = sa[3]
@@ -496,7 +497,7 @@ class LlamaEngine:
             g = st.unit_grads(1 + i)
             if i < self.recompute_layers:
                 _, saved = self._layer_fwd(w, ckpt[i], B, S, keep=True,
-                                           attn_saved=saved_all[i])
+                                           attn_saved=saved_all[i], need_out=False)
                 saved_all[i] = None
             else:
                 saved = saved_all[i]

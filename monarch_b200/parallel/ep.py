@@ -283,7 +283,8 @@ class MoEEngine(LlamaEngine):
             wts = top_p / top_p.sum(-1, keepdim=True)
         return top_i, wts
 
-    def _mlp_fwd(self, w, x2, keep):
+    def _mlp_fwd(self, w, x2, keep, need_out=True):
+        # the exchange runs as a whole on every rank, whether its result is needed or not
         h2, rstd2 = ops.rmsnorm_fwd(x2, w["mlp_norm"], self.cfg.eps)
         top_i, wts = self._route(h2, w["router"], False)
         y, sv = self.ep.forward(h2, top_i.to(torch.int32).contiguous(), wts.contiguous(),
