@@ -90,14 +90,6 @@ __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------------ dK, dV
-__device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes,
-                                             uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-
 // The operand that the last MMA of a step still reads has three stages (its buffer comes free
 // only two MMAs before the next tile in it is needed), the other one two.
 constexpr int AB_ST3 = 3;

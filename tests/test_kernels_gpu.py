@@ -247,3 +247,90 @@ def test_gemm_tile_choice(M, N, K_, a_mn, b_mn):
     first = wide[:, :N].clone()
     ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=wide[:, :N], accumulate=True)
     assert _rel(wide[:, :N], ref - r.double() + first.double()) < 2.5e-3
+
+
+# one row, rows that leave the last block short, more rows than a ring has stages and than there
+# are blocks; d: one chunk, a remainder of a warp's chunk, both sides of every variant's limit
+@pytest.mark.parametrize("rows,d", [(1, 8), (5, 264), (3000, 512), (77, 2048), (700, 2056),
+                                    (1201, 4096), (19, 4104), (333, 5120), (2, 8192)])
+def test_rmsnorm_row_lengths(rows, d):
+    torch.manual_seed(1)
+    x = torch.randn(rows, d, device="cuda", dtype=bf16)
+    w = (1 + 0.1 * torch.randn(d, device="cuda")).to(bf16)
+    dy = torch.randn(rows, d, device="cuda", dtype=bf16)
+    dres = torch.randn(rows, d, device="cuda", dtype=bf16)
+    y, rstd = ops.rmsnorm_fwd(x, w, 1e-5)
+    yr, rstdr = R.rmsnorm_fwd(x.double(), w.double(), 1e-5)
+    # bf16 results are off by their rounding (1.7e-3 in the 2-norm), rstd by fp32 sums
+    assert _rel(y, yr) < 3e-3 and _rel(rstd, rstdr) < 1e-6
+    for res in (dres, None):
+        dw = torch.zeros(d, device="cuda", dtype=bf16)
+        dx = ops.rmsnorm_bwd(dy, x, w, rstd, dw, dres=res)
+        dxr, dwr = R.rmsnorm_bwd(dy, x, w, rstdr.float())
+        assert _rel(dx, dxr if res is None else dxr + res.float()) < 3e-3
+        assert _rel(dw, dwr) < 3e-3
+
+
+def test_rmsnorm_fwd_longer_than_registers():
+    x = torch.randn(3, 8200, device="cuda", dtype=bf16)
+    w = torch.ones(8200, device="cuda", dtype=bf16)
+    y, _ = ops.rmsnorm_fwd(x, w, 1e-5)
+    assert _rel(y, R.rmsnorm_fwd(x, w, 1e-5)[0]) < 3e-3
+
+
+# head sizes with 1, 4, 8, 32 threads per head and two that take the general kernel; heads that
+# leave the last batch of a thread short
+@pytest.mark.parametrize("hd,heads", [(16, 3), (64, 40), (128, 1), (128, 41), (512, 2), (1024, 2), (48, 5)])
+@pytest.mark.parametrize("rows,S", [(7, 4), (130, 64)])
+def test_rope_head_sizes(hd, heads, rows, S):
+    torch.manual_seed(2)
+    cos, sin = R.rope_tables(S, hd, 10000.0, device="cuda")
+    x = torch.randn(rows, heads * hd + 16, device="cuda", dtype=bf16)
+    before = x.clone()
+    for inverse in (False, True):
+        y = before.clone()
+        ops.rope_(y, cos, sin, S, heads, hd, inverse=inverse)
+        ref = R.rope(before[:, : heads * hd].float().reshape(rows, heads, hd), cos, sin, S, inverse)
+        assert _rel(y[:, : heads * hd], ref.reshape(rows, -1)) < 3e-3
+        assert torch.equal(y[:, heads * hd:], before[:, heads * hd:])
+
+
+@pytest.mark.parametrize("rows,F", [(1, 8), (3, 264), (5, 2048), (2, 2056)])
+def test_swiglu_row_lengths(rows, F):
+    gu = torch.randn(rows, 2 * F, device="cuda", dtype=bf16)
+    dh = torch.randn(rows, F, device="cuda", dtype=bf16)
+    assert _rel(ops.swiglu_fwd(gu), R.swiglu_fwd(gu)) < 3e-3
+    assert _rel(ops.swiglu_bwd(gu, dh), R.swiglu_bwd(gu, dh)) < 3e-3
+
+
+# both sides of the block sizes' limits, and lengths with a scalar remainder
+@pytest.mark.parametrize("V", [8, 513, 4096, 4100, 65536, 65541, 100003])
+def test_cross_entropy_vocabularies(V):
+    torch.manual_seed(3)
+    rows, ld = 5, (V + 15) // 8 * 8
+    wide = (3 * torch.randn(rows, ld, device="cuda")).to(bf16)
+    rest = wide[:, V:].clone()
+    tg = torch.tensor([0, V - 1, V // 2, 1, 7], device="cuda")
+    lr, gr = R.cross_entropy(wide[:, :V], tg, 0.25)
+    loss = ops.cross_entropy_(wide[:, :V], tg, 0.25)
+    assert torch.allclose(loss, lr, atol=2e-4, rtol=1e-4)
+    assert _rel(wide[:, :V], gr) < 3e-3
+    assert torch.equal(wide[:, V:], rest)
+
+
+# 16-byte reductions (d % 8 == 0), pairs for the others; every token once, then many of one
+@pytest.mark.parametrize("d", [8, 250, 2056])
+def test_embedding_bwd_widths(d):
+    torch.manual_seed(4)
+    ids = torch.randperm(300, device="cuda")[:200]
+    dout = torch.randn(200, d, device="cuda", dtype=bf16)
+    base = torch.randn(300, d, device="cuda", dtype=bf16)
+    dt = base.clone()
+    ops.embedding_bwd_(dout, ids, dt)
+    ref = base.clone()
+    ref[ids] += dout
+    assert torch.equal(dt, ref)
+    one = torch.zeros(3, d, device="cuda", dtype=bf16)
+    ops.embedding_bwd_(torch.ones(100, d, device="cuda", dtype=bf16),
+                       torch.full((100,), 1, device="cuda"), one)
+    assert (one[1] == 100).all() and one[0].abs().max() == 0 and one[2].abs().max() == 0
