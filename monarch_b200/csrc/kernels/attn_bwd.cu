@@ -25,8 +25,13 @@
 //                                                dS(t+1) under dV(t+1) and S(t+2)
 //   dQ:     S(t+1) dP(t+1) dQ(t) ...             (dP has two buffers here, S is free again as
 //                                                soon as the warps hold it in registers)
-// B1 S8192 32q/8kv hd128: dK/dV 1361 -> 853 us, dQ 1223 -> 616 us against the 64-row steps;
-// B2 S4096 32q/8kv hd64: 551 -> 383 us and 518 -> 281 us.
+// dK/dV is bound by the chain P(t) -> dV(t) -> S(t+1) -> P(t+1), as P lies over S: P is handed
+// over in halves, so that dV starts under the second half of the exponentials; at hd 64 TMEM
+// has room for P beside S and S(t+1) is issued as soon as S(t) is in registers.
+// B1 S8192 32q/8kv hd128, dK/dV + dQ + delta: 2638 us with 64-row steps, 1564 with 128-row steps,
+// 1518 with the halves: 7 MMAs per block pair at 1.35 PFLOP/s, which is what the chip sustains
+// under its power cap (exponentials on the FMA pipe took 6 % off the cycles and as much off the
+// clock).  B2 S4096 32q/8kv hd64: 1120, 703, 641 us.
 //
 // Warp roles (576 threads): 0 TMA producer, 1 MMA issuer, 2-17 compute/epilogue; warps w,
 // w+4, w+8, w+12 share a TMEM lane quadrant and split the 128 columns of a tile in quarters
@@ -112,7 +117,7 @@ struct DkvBars {
   uint64_t q_full[AB_ST3], q_empty[AB_ST3];
   uint64_t do_full[AB_ST2], do_empty[AB_ST2];
   uint64_t ld_full[AB_ST2], ld_empty[AB_ST2];
-  uint64_t s_full, dp_full, p_ready, ds_ready, acc_done;
+  uint64_t s_full, s_free, dp_full, p_half, p_ready, ds_ready, acc_done;
   uint32_t tmem_base;
   volatile int abort_word;
 };
@@ -137,16 +142,28 @@ __device__ __forceinline__ void mma_scores(uint32_t d_tmem, uint32_t sa, uint32_
              umma_smem_desc_sw128(sb + off, 16, 1024), idesc, kk > 0 ? 1u : 0u);
   }
 }
-// D[128, HD] (+)= A B over 128 rows: A bf16 in TMEM (quarters of 16 columns every 32), B MN-major
+// D[128, HD] (+)= A B over 128 rows: A bf16 in TMEM (quarters of 16 columns), B MN-major
+template <int HD, int QUARTER = 32>
+__device__ __forceinline__ void mma_grad_half(uint32_t d_tmem, uint32_t a_tmem, uint32_t sb,
+                                              int half, bool accumulate) {
+  // one half of every quarter
+  constexpr uint32_t idesc = umma_idesc_bf16(AB_T, HD, 0, 1);
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    umma_f16_ts(d_tmem, a_tmem + c * QUARTER + half * 8,
+                umma_smem_desc_sw128(sb + (2 * c + half) * 2048, AB_T * 128, 1024), idesc,
+                (accumulate || c > 0) ? 1u : 0u);
+}
 template <int HD>
 __device__ __forceinline__ void mma_grad(uint32_t d_tmem, uint32_t a_tmem, uint32_t sb,
                                          bool accumulate) {
-  constexpr uint32_t idesc = umma_idesc_bf16(AB_T, HD, 0, 1);
-#pragma unroll
-  for (int kk = 0; kk < AB_T / 16; ++kk)
-    umma_f16_ts(d_tmem, a_tmem + (kk >> 1) * 32 + (kk & 1) * 8,
-                umma_smem_desc_sw128(sb + kk * 2048, AB_T * 128, 1024), idesc,
-                (accumulate || kk > 0) ? 1u : 0u);
+  mma_grad_half<HD>(d_tmem, a_tmem, sb, 0, accumulate);
+  mma_grad_half<HD>(d_tmem, a_tmem, sb, 1, true);
+}
+
+__device__ __forceinline__ float2 exp2_pair(uint64_t x) {
+  const float2 e = unpack_f32x2(x);
+  return make_float2(ex2_approx(e.x), ex2_approx(e.y));
 }
 
 template <int HD>
@@ -192,7 +209,9 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
       mbar_init(&bars->ld_empty[s], 1);
     }
     mbar_init(&bars->s_full, 1);
+    mbar_init(&bars->s_free, 16);
     mbar_init(&bars->dp_full, 1);
+    mbar_init(&bars->p_half, 16);
     mbar_init(&bars->p_ready, 16);
     mbar_init(&bars->ds_ready, 16);
     mbar_init(&bars->acc_done, 1);
@@ -208,8 +227,12 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile int* abort_word = &bars->abort_word;
-  // TMEM columns: S^T/P^T at 0, dP^T/dS^T at 128, dV at 256, dK at 256 + HD
-  constexpr uint32_t kColDP = 128, kColDV = 256, kColDK = 256 + HD;
+  // TMEM columns: S^T at 0, dP^T/dS^T at 128, dV at 256, dK at 256 + HD; P^T over S^T at hd 128.
+  // At hd 64 P^T(t) has 64 columns of its own at 384 + (t & 1) * 64: S(t) was issued behind
+  // dV(t-2), so a warp that has S(t) may overwrite P(t-2).
+  constexpr bool kOwnP = HD == 64;
+  constexpr uint32_t kColDP = 128, kColDV = 256, kColDK = 256 + HD, kColP = kOwnP ? 384 : 0;
+  constexpr int kQuarterP = kOwnP ? 16 : 32;   // columns from one quarter of P to the next
 
   if (warp == 0) {
     if (elect_one()) {
@@ -261,23 +284,36 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
         mma_scores<HD>(tmem_base + kColDP, sv, sdo);
         umma_commit(&bars->dp_full);
       }
+      const auto next_s = [&](int t) -> bool {   // S(t + 1)
+        const int n3 = (t + 1) % AB_ST3;
+        if (!mbar_wait(&bars->q_full[n3], (uint32_t)((t + 1) / AB_ST3) & 1, abort_word, p.status))
+          return false;
+        tc_fence_after();
+        mma_scores<HD>(tmem_base, sk, sq + n3 * SM::kTile);
+        umma_commit(&bars->s_full);
+        return true;
+      };
       for (int t = 0; ok && t < nsteps; ++t) {
-        const int q3 = t % AB_ST3, d2 = t % AB_ST2;
-        const int nq3 = (t + 1) % AB_ST3, nd2 = (t + 1) % AB_ST2;
+        const int q3 = t % AB_ST3, d2 = t % AB_ST2, nd2 = (t + 1) % AB_ST2;
         const uint32_t par = (uint32_t)t & 1;
         const bool more = t + 1 < nsteps;
+        if (kOwnP && more) {
+          ok = mbar_wait(&bars->s_free, par, abort_word, p.status) && next_s(t);
+          if (!ok) break;
+        }
+        ok = mbar_wait(&bars->p_half, par, abort_word, p.status);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t tp = tmem_base + kColP + (kOwnP ? (t & 1) * 64 : 0);
+        mma_grad_half<HD, kQuarterP>(tmem_base + kColDV, tp, sdo + d2 * SM::kTile, 0, t > 0);
         ok = mbar_wait(&bars->p_ready, par, abort_word, p.status);
         if (!ok) break;
         tc_fence_after();
-        mma_grad<HD>(tmem_base + kColDV, tmem_base, sdo + d2 * SM::kTile, t > 0);
+        mma_grad_half<HD, kQuarterP>(tmem_base + kColDV, tp, sdo + d2 * SM::kTile, 1, true);
         umma_commit(&bars->do_empty[d2]);
-        if (more) {   // overwrites P(t): ordered behind dV(t) on the tensor pipe
-          ok = mbar_wait(&bars->q_full[nq3], (uint32_t)((t + 1) / AB_ST3) & 1, abort_word,
-                         p.status);
+        if (!kOwnP && more) {   // overwrites P(t): ordered behind dV(t) on the tensor pipe
+          ok = next_s(t);
           if (!ok) break;
-          tc_fence_after();
-          mma_scores<HD>(tmem_base, sk, sq + nq3 * SM::kTile);
-          umma_commit(&bars->s_full);
         }
         ok = mbar_wait(&bars->ds_ready, par, abort_word, p.status);
         if (!ok) break;
@@ -320,32 +356,43 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
       uint32_t sv[32];
       tmem_ld_32x32b_x32(t_st, sv);
       tmem_ld_wait();
+      if (kOwnP) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->s_free);
+      }
       uint32_t pk[16];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 l4 = *reinterpret_cast<const float4*>(sl + 4 * i);
-        const float2 e0 = unpack_f32x2(
-            fma_f32x2(pack_f32x2(__uint_as_float(sv[4 * i]), __uint_as_float(sv[4 * i + 1])), c2,
-                      mul_f32x2(pack_f32x2(l4.x, l4.y), nlog2e)));
-        const float2 e1 = unpack_f32x2(
-            fma_f32x2(pack_f32x2(__uint_as_float(sv[4 * i + 2]), __uint_as_float(sv[4 * i + 3])),
-                      c2, mul_f32x2(pack_f32x2(l4.z, l4.w), nlog2e)));
-        float pv[4] = {ex2_approx(e0.x), ex2_approx(e0.y), ex2_approx(e1.x), ex2_approx(e1.y)};
-        if (sub == 0) {
+      for (int half = 0; half < 2; ++half) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (part * 32 + 4 * i + e < r) pv[e] = 0.f;  // query before the key position
+        for (int i = half * 4; i < half * 4 + 4; ++i) {
+          const float4 l4 = *reinterpret_cast<const float4*>(sl + 4 * i);
+          const float2 e0 = exp2_pair(
+              fma_f32x2(pack_f32x2(__uint_as_float(sv[4 * i]), __uint_as_float(sv[4 * i + 1])),
+                        c2, mul_f32x2(pack_f32x2(l4.x, l4.y), nlog2e)));
+          const float2 e1 = exp2_pair(
+              fma_f32x2(pack_f32x2(__uint_as_float(sv[4 * i + 2]), __uint_as_float(sv[4 * i + 3])),
+                        c2, mul_f32x2(pack_f32x2(l4.z, l4.w), nlog2e)));
+          float pv[4] = {e0.x, e0.y, e1.x, e1.y};
+          if (sub == 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (part * 32 + 4 * i + e < r) pv[e] = 0.f;  // query before the key position
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sv[4 * i + e] = __float_as_uint(pv[e]);
+          pk[2 * i] = pack_bf16x2(pv[0], pv[1]);
+          pk[2 * i + 1] = pack_bf16x2(pv[2], pv[3]);
         }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sv[4 * i + e] = __float_as_uint(pv[e]);
-        pk[2 * i] = pack_bf16x2(pv[0], pv[1]);
-        pk[2 * i + 1] = pack_bf16x2(pv[2], pv[3]);
+        const uint32_t t_p = tmem_base + lane_off + kColP + part * kQuarterP +
+                             (kOwnP ? (t & 1) * 64 : 0);
+        tmem_st_32x32b_x8(t_p + half * 8,
+                          *reinterpret_cast<const uint32_t(*)[8]>(&pk[half * 8]));
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(half == 0 ? &bars->p_half : &bars->p_ready);
       }
-      tmem_st_32x32b_x16(t_st, pk);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->p_ready);
       ok = mbar_wait(&bars->dp_full, par, abort_word, p.status);
       if (!ok) break;
       tc_fence_after();
@@ -574,10 +621,11 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
       if (lane == 0) mbar_arrive(&bars->s_free);
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        const float2 x = unpack_f32x2(fma_f32x2(
-            pack_f32x2(__uint_as_float(sv[2 * e]), __uint_as_float(sv[2 * e + 1])), c2, nl2));
-        sv[2 * e] = __float_as_uint(ex2_approx(x.x));
-        sv[2 * e + 1] = __float_as_uint(ex2_approx(x.y));
+        const float2 x = exp2_pair(
+            fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * e]), __uint_as_float(sv[2 * e + 1])), c2,
+                      nl2));
+        sv[2 * e] = __float_as_uint(x.x);
+        sv[2 * e + 1] = __float_as_uint(x.y);
       }
       if (t == i) {   // the diagonal block
 #pragma unroll

@@ -112,3 +112,20 @@ def test_attention_backward(B, S, Hq, Hkv, hd):
     assert _rel(dqkv[:, :n_q], ref[:, :n_q]) < 2e-2, ("dq", _rel(dqkv[:, :n_q], ref[:, :n_q]))
     assert _rel(dqkv[:, n_q:n_q + n_k], ref[:, n_q:n_q + n_k]) < 2e-2, "dk"
     assert _rel(dqkv[:, n_q + n_k:], ref[:, n_q + n_k:]) < 2e-2, "dv"
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,hd", [(2, 4096, 16, 4, 64), (1, 4096, 16, 4, 128)])
+def test_attention_is_reproducible(B, S, Hq, Hkv, hd):
+    """No atomics and no order that depends on timing: repeated passes give the same bits, which
+    a missing wait between the tensor pipe and the softmax warps would break on many CTAs."""
+    from monarch_b200 import ops
+    torch.manual_seed(3)
+    qkv = torch.randn(B * S, (Hq + 2 * Hkv) * hd, device="cuda").to(bf16)
+    do = torch.randn(B * S, Hq * hd, device="cuda").to(bf16)
+    first = None
+    for _ in range(4):
+        o, ctx = ops.attention_fwd(qkv, B, S, Hq, Hkv, hd)
+        got = (o, ctx.lse, ops.attention_bwd(ctx, do))
+        if first is None:
+            first = got
+        assert all(torch.equal(a, b) for a, b in zip(first, got))
