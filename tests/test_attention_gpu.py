@@ -129,3 +129,21 @@ def test_attention_is_reproducible(B, S, Hq, Hkv, hd):
         if first is None:
             first = got
         assert all(torch.equal(a, b) for a, b in zip(first, got))
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_backward_with_an_output_that_is_not_16_byte_aligned(hd):
+    """delta reads the forward's output with 16-byte loads only where it may."""
+    from monarch_b200 import ops
+    torch.manual_seed(4)
+    B, S, Hq, Hkv = 1, 256, 4, 2
+    qkv = torch.randn(B * S, (Hq + 2 * Hkv) * hd, device="cuda").to(bf16)
+    do = torch.randn(B * S, Hq * hd, device="cuda").to(bf16)
+    o, ctx = ops.attention_fwd(qkv, B, S, Hq, Hkv, hd)
+    want = ops.attention_bwd(ctx, do)
+    shifted = torch.empty(B * S, Hq * hd + 8, dtype=bf16, device="cuda")[:, 2: 2 + Hq * hd]
+    shifted.copy_(o)
+    _, ctx2 = ops.attention_ctx_from_saved(qkv, (shifted, ctx.lse), B, S, Hq, Hkv, hd)
+    do2 = torch.empty(B * S, Hq * hd + 8, dtype=bf16, device="cuda")[:, :Hq * hd]
+    do2.copy_(do)
+    assert torch.equal(ops.attention_bwd(ctx2, do2), want)
