@@ -42,6 +42,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "launch.cuh"
 #include "mb200.h"
 #include "ptx.cuh"
 
@@ -84,6 +85,8 @@ __global__ void __launch_bounds__(256)
     attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                       float* __restrict__ delta, int S, int Hq, int ld_o, int ld_do) {
   constexpr int LANES = HD / 8, ROWS = 256 / LANES;   // rows of a block: ROWS * AB_DELTA_U
+  dep_launch();
+  dep_wait();
   const int h = (int)(blockIdx.x % Hq);
   const int lane = (int)threadIdx.x % LANES;
   const long long row0 =
@@ -248,6 +251,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile int* abort_word = &bars->abort_word;
+  dep_wait();
   // TMEM columns: S^T at 0, dP^T/dS^T at 128, dV at 256, dK at 256 + HD; P^T over S^T at hd 128.
   // At hd 64 P^T(t) has 64 columns of its own at 384 + (t & 1) * 64: S(t) was issued behind
   // dV(t-2), so a warp that has S(t) may overwrite P(t-2).
@@ -551,6 +555,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile int* abort_word = &bars->abort_word;
+  dep_wait();
   // TMEM columns: S at 0, dP/dS of step t at 128 + (t&1)*128, dQ at 384
   constexpr uint32_t kColDP = 128, kColDQ = 384;
 
@@ -733,13 +738,11 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
   if (!r) r = make_tmap_bf16_2d(&tdo, dout, (uint64_t)p.Hq * HD, T, ld_do, 64, AB_T);
   if (r) return 1000 - r;
   const int n_blk = p.S / AB_T;
-  attn_bwd_dkv_kernel<HD><<<dim3(n_blk * p.Hkv * p.B), AB_THREADS, AbSmem<HD>::kTotal, st>>>(
-      tq, tk, tv, tdo, p);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_dep(attn_bwd_dkv_kernel<HD>, n_blk * p.Hkv * p.B, AB_THREADS,
+                                   AbSmem<HD>::kTotal, st, tq, tk, tv, tdo, p);
   if (e != cudaSuccess) return (int)e;
-  attn_bwd_dq_kernel<HD><<<dim3(n_blk, p.Hq, p.B), AB_THREADS, AbSmem<HD>::kTotal, st>>>(
-      tq, tk, tv, tdo, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(attn_bwd_dq_kernel<HD>, dim3(n_blk, p.Hq, p.B), AB_THREADS,
+                         AbSmem<HD>::kTotal, st, tq, tk, tv, tdo, p);
 }
 
 }  // namespace mb200
@@ -766,9 +769,9 @@ extern "C" int mb200_attn_bwd(const void* q, const void* k, const void* v, const
       hd == 128 ? (vec ? attn_delta_kernel<128, true> : attn_delta_kernel<128, false>)
                 : (vec ? attn_delta_kernel<64, true> : attn_delta_kernel<64, false>);
   const long long rows = (long long)B * S;
-  delta_kernel<<<(unsigned)(rows / (hd == 128 ? 64 : 128) * Hq), 256, 0, st>>>(
-      ob, db, delta, S, Hq, ld_o, ld_o);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e =
+      launch_dep(delta_kernel, (unsigned)(rows / (hd == 128 ? 64 : 128) * Hq), 256, 0, st, ob, db,
+                 delta, S, Hq, ld_o, ld_o);
   if (e != cudaSuccess) return (int)e;
   AttBwdParams p{};
   p.lse = lse;

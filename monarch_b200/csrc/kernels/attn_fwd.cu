@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "launch.cuh"
 #include "mb200.h"
 #include "ptx.cuh"
 
@@ -121,6 +122,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
   const int jmax = last[1] > last[0] ? last[1] : last[0];
   const int row_base = b * p.S;
 
+
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
     for (int s = 0; s < ATT_KV_STAGES; ++s) {
@@ -148,6 +150,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   volatile int* abort_word = &bars->abort_word;
+  dep_wait();
   // TMEM columns: S of slot s at s*128, O at 256 + s*HD, P over S (hd 128) or at 384 + s*64
   constexpr bool kOwnP = HD == 64;
   constexpr uint32_t kColO = 256, kColP = kOwnP ? 384 : 0, kStrideP = kOwnP ? 64 : 128;
@@ -420,8 +423,7 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const At
     grid = dim3(n_qblk, p.Hq / 2, p.B);
   else
     grid = dim3((n_qblk + 1) / 2, p.Hq, p.B);
-  attn_fwd_kernel<HD><<<grid, ATT_THREADS, SM::kTotal, st>>>(tq, tk, tv, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(attn_fwd_kernel<HD>, grid, ATT_THREADS, SM::kTotal, st, tq, tk, tv, p);
 }
 
 }  // namespace mb200

@@ -5,6 +5,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "mb200.h"
 #include "ptx.cuh"
 
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(128)
     rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x,
                            const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                            float* __restrict__ rstd, int rows, int d, float eps) {
+  dep_wait();
   __shared__ float red[4];
   const int warp = threadIdx.x >> 5;
   const int t = (int)threadIdx.x % (32 * WPR);   // place in the row's group of warps
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(128)
 __global__ void __launch_bounds__(256)
     rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                        __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int d, float eps) {
+  dep_wait();
   __shared__ float red[33];
   const size_t row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * d;
@@ -178,6 +181,9 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
     abort_word = 0;
     mbar_fence_init();
+  }
+  dep_wait();
+  if (threadIdx.x == 0) {
     for (int it = 0; it < stages && it < n; ++it) fill(it);
   }
   float acc[NCH][8];
@@ -263,6 +269,7 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
 __global__ void __launch_bounds__(1024)
     rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int nblocks, int d,
                              __nv_bfloat16* __restrict__ dw, int accumulate) {
+  dep_wait();
   __shared__ float sh[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -298,9 +305,8 @@ static int launch_rmsnorm_bwd_t(int nb, const __nv_bfloat16* dy, const __nv_bflo
   const int stage = (RES ? 3 : 2) * d * 2;
   int stages = kRing / stage;
   if (stages > RMS_BWD_MAX_STAGES) stages = RMS_BWD_MAX_STAGES;
-  rmsnorm_bwd_kernel<NT, NCH, RES><<<nb, NT, stages * stage, st>>>(dy, x, w, rstd, dres, dx,
-                                                                  dw_partial, rows, d, stages);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(rmsnorm_bwd_kernel<NT, NCH, RES>, nb, NT, stages * stage, st, dy, x, w,
+                         rstd, dres, dx, dw_partial, rows, d, stages);
 }
 
 // Launches the backward pair: nb row-striding blocks (fewer where one block fills an SM), then
@@ -326,8 +332,8 @@ static int launch_rmsnorm_bwd(int nb, const __nv_bfloat16* dy, const __nv_bfloat
     rc = MB200_RMS_BWD(512, 2);
 #undef MB200_RMS_BWD
   if (rc) return rc;
-  rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, 1024, 0, st>>>(dw_partial, nb, d, dw, dw_accumulate);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(rmsnorm_dw_reduce_kernel, (d + 31) / 32, 1024, 0, st, dw_partial, nb, d,
+                         dw, dw_accumulate);
 }
 
 // --------------------------------------------------------------------- RoPE --
@@ -340,6 +346,7 @@ __global__ void __launch_bounds__(256)
     rope_row_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                     const float* __restrict__ sin_t, int rows, int seq_len, int n_rot_heads,
                     int log2_hd, int row_stride, int inverse) {
+  dep_wait();
   const int hd = 1 << log2_hd, half = hd >> 1, per_head = hd >> 4;
   const int log2_row = log2_hd - 1;   // hd / 2 = 8 * per_head threads per row
   const int row = ((int)blockIdx.x << (8 - log2_row)) + ((int)threadIdx.x >> log2_row);
@@ -394,6 +401,7 @@ __global__ void __launch_bounds__(256)
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, long long total, int seq_len,
                             int n_rot_heads, int hd, int row_stride, int inverse) {
+  dep_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const int half = hd >> 1;
@@ -429,6 +437,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
 // the forward a fifth of its time: 8192x14336 133.6 -> 113 us, backward 181 -> 178 us).
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                   __nv_bfloat16* __restrict__ h, int F) {
+  dep_wait();
   const size_t row = blockIdx.x;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
   if (c >= F) return;
@@ -443,6 +452,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                   const __nv_bfloat16* __restrict__ dh,
                                   __nv_bfloat16* __restrict__ dgu, int F) {
+  dep_wait();
   const size_t row = blockIdx.x;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
   if (c >= F) return;
@@ -473,6 +483,7 @@ template <int CE_THREADS>
 __global__ void __launch_bounds__(CE_THREADS, 2048 / CE_THREADS)
     cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
                          float* __restrict__ loss_rows, int V, int ld, float grad_scale) {
+  dep_wait();
   __shared__ float red_m[CE_THREADS / 32];
   __shared__ float red_s[CE_THREADS / 32];
   __shared__ float bc[2];
@@ -571,6 +582,7 @@ __global__ void adamw_kernel(float* __restrict__ p, float* __restrict__ m, float
                              const void* __restrict__ g, __nv_bfloat16* __restrict__ pb, int64_t n,
                              int g_bf16, float lr, float beta1, float beta2, float eps, float wd,
                              float inv_bc1, float inv_sqrt_bc2, float grad_scale) {
+  dep_wait();
   const int64_t i4 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
   float pv[4], mv[4], vv[4], gv[4];
@@ -634,6 +646,7 @@ __global__ void adamw_kernel(float* __restrict__ p, float* __restrict__ m, float
 __global__ void embedding_fwd_kernel(const __nv_bfloat16* __restrict__ table,
                                      const int64_t* __restrict__ ids,
                                      __nv_bfloat16* __restrict__ out, long long total, int d) {
+  dep_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const int per_row = d >> 3;
@@ -648,6 +661,7 @@ __global__ void embedding_fwd_kernel(const __nv_bfloat16* __restrict__ table,
 __global__ void embedding_bwd_vec_kernel(const __nv_bfloat16* __restrict__ dout,
                                          const int64_t* __restrict__ ids,
                                          __nv_bfloat16* __restrict__ dtable, int d) {
+  dep_wait();
   const size_t row = blockIdx.x;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
   if (c >= d) return;
@@ -660,6 +674,7 @@ __global__ void embedding_bwd_vec_kernel(const __nv_bfloat16* __restrict__ dout,
 __global__ void embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dout,
                                      const int64_t* __restrict__ ids,
                                      __nv_bfloat16* __restrict__ dtable, long long total, int d) {
+  dep_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const int per_row = d >> 1;
@@ -672,6 +687,7 @@ __global__ void embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dout,
 
 __global__ void sumsq_kernel(const void* __restrict__ x, int64_t n, int is_bf16,
                              float* __restrict__ out) {
+  dep_wait();
   __shared__ float red[33];
   float s = 0.f;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -701,22 +717,16 @@ extern "C" int mb200_rmsnorm_fwd(const void* x, const void* w, void* y, float* r
   if (rows <= 0) return 0;
   if (d % 8) return 1001;
 #define MB200_RMS_FWD(NV, WPR)                                                              \
-  rmsnorm_fwd_row_kernel<NV, WPR><<<blocks_for(rows, 4 / WPR), 128, 0, ST(stream)>>>(       \
-      CBF(x), CBF(w), BF(y), rstd, rows, d, eps)
-  if (d <= 512)
-    MB200_RMS_FWD(2, 1);
-  else if (d <= 1024)
-    MB200_RMS_FWD(4, 1);
-  else if (d <= 2048)
-    MB200_RMS_FWD(8, 1);
-  else if (d <= 4096)
-    MB200_RMS_FWD(8, 2);
-  else if (d <= 8192)
-    MB200_RMS_FWD(8, 4);
-  else
-    rmsnorm_fwd_kernel<<<rows, 256, 0, ST(stream)>>>(CBF(x), CBF(w), BF(y), rstd, d, eps);
+  return (int)launch_dep(rmsnorm_fwd_row_kernel<NV, WPR>, blocks_for(rows, 4 / WPR), 128, 0, \
+                         ST(stream), CBF(x), CBF(w), BF(y), rstd, rows, d, eps)
+  if (d <= 512) MB200_RMS_FWD(2, 1);
+  if (d <= 1024) MB200_RMS_FWD(4, 1);
+  if (d <= 2048) MB200_RMS_FWD(8, 1);
+  if (d <= 4096) MB200_RMS_FWD(8, 2);
+  if (d <= 8192) MB200_RMS_FWD(8, 4);
 #undef MB200_RMS_FWD
-  return (int)cudaGetLastError();
+  return (int)launch_dep(rmsnorm_fwd_kernel, rows, 256, 0, ST(stream), CBF(x), CBF(w), BF(y), rstd,
+                         d, eps);
 }
 
 extern "C" int mb200_rmsnorm_bwd_blocks(int rows) {
@@ -740,15 +750,13 @@ extern "C" int mb200_rope_inplace(void* qkv, const float* cos_t, const float* si
   if (rows <= 0) return 0;
   if (hd % 16 || row_stride % 8) return 1001;
   if (hd <= 512 && (hd & (hd - 1)) == 0 && aligned16(cos_t) && aligned16(sin_t)) {
-    rope_row_kernel<<<blocks_for(rows, 32 / (hd / 16)), 256, 0, ST(stream)>>>(
-        BF(qkv), cos_t, sin_t, rows, seq_len, n_rot_heads, __builtin_ctz(hd), row_stride, inverse);
-    return (int)cudaGetLastError();
+    return (int)launch_dep(rope_row_kernel, blocks_for(rows, 32 / (hd / 16)), 256, 0, ST(stream),
+                           BF(qkv), cos_t, sin_t, rows, seq_len, n_rot_heads, __builtin_ctz(hd),
+                           row_stride, inverse);
   }
   const long long total = (long long)rows * n_rot_heads * (hd / 16);
-  rope_kernel<<<blocks_for(total, 256), 256, 0, ST(stream)>>>(BF(qkv), cos_t, sin_t, total,
-                                                              seq_len, n_rot_heads, hd, row_stride,
-                                                              inverse);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(rope_kernel, blocks_for(total, 256), 256, 0, ST(stream), BF(qkv), cos_t,
+                         sin_t, total, seq_len, n_rot_heads, hd, row_stride, inverse);
 }
 
 extern "C" int mb200_swiglu_fwd(const void* gu, void* h, int rows, int F, void* stream) {
@@ -756,8 +764,8 @@ extern "C" int mb200_swiglu_fwd(const void* gu, void* h, int rows, int F, void* 
   if (F % 8) return 1001;
   if (F <= 0) return 0;
   const int nt = row_threads(F / 8);
-  swiglu_fwd_kernel<<<dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream)>>>(CBF(gu), BF(h), F);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(swiglu_fwd_kernel, dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream),
+                         CBF(gu), BF(h), F);
 }
 extern "C" int mb200_swiglu_bwd(const void* gu, const void* dh, void* dgu, int rows, int F,
                                 void* stream) {
@@ -765,9 +773,8 @@ extern "C" int mb200_swiglu_bwd(const void* gu, const void* dh, void* dgu, int r
   if (F % 8) return 1001;
   if (F <= 0) return 0;
   const int nt = row_threads(F / 8);
-  swiglu_bwd_kernel<<<dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream)>>>(CBF(gu), CBF(dh),
-                                                                             BF(dgu), F);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(swiglu_bwd_kernel, dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream),
+                         CBF(gu), CBF(dh), BF(dgu), F);
 }
 
 extern "C" int mb200_cross_entropy_fwd_bwd(void* logits, const int64_t* targets, float* loss_rows,
@@ -775,17 +782,13 @@ extern "C" int mb200_cross_entropy_fwd_bwd(void* logits, const int64_t* targets,
                                            void* stream) {
   if (rows <= 0) return 0;
   if (ld % 8) return 1001;
-#define MB200_CE(NT)                                                                         \
-  cross_entropy_kernel<NT><<<rows, NT, 0, ST(stream)>>>(BF(logits), targets, loss_rows, V, ld, \
-                                                        grad_scale)
-  if (V <= 4096)
-    MB200_CE(128);
-  else if (V <= 65536)
-    MB200_CE(512);
-  else
-    MB200_CE(1024);
+#define MB200_CE(NT)                                                                      \
+  return (int)launch_dep(cross_entropy_kernel<NT>, rows, NT, 0, ST(stream), BF(logits), targets, \
+                         loss_rows, V, ld, grad_scale)
+  if (V <= 4096) MB200_CE(128);
+  if (V <= 65536) MB200_CE(512);
+  MB200_CE(1024);
 #undef MB200_CE
-  return (int)cudaGetLastError();
 }
 
 extern "C" int mb200_adamw(float* p, float* m, float* v, const void* g, void* p_bf16, int64_t n,
@@ -795,10 +798,9 @@ extern "C" int mb200_adamw(float* p, float* m, float* v, const void* g, void* p_
   const double bc1 = 1.0 - pow((double)beta1, (double)step);
   const double bc2 = 1.0 - pow((double)beta2, (double)step);
   const long long nthreads = (n + 3) / 4;
-  adamw_kernel<<<blocks_for(nthreads, 256), 256, 0, ST(stream)>>>(
-      p, m, v, g, BF(p_bf16), n, g_bf16, lr, beta1, beta2, eps, wd, (float)(1.0 / bc1),
-      (float)(1.0 / sqrt(bc2)), grad_scale);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(adamw_kernel, blocks_for(nthreads, 256), 256, 0, ST(stream), p, m, v, g,
+                         BF(p_bf16), n, g_bf16, lr, beta1, beta2, eps, wd, (float)(1.0 / bc1),
+                         (float)(1.0 / sqrt(bc2)), grad_scale);
 }
 
 extern "C" int mb200_embedding_fwd(const void* table, const int64_t* ids, void* out, int rows,
@@ -806,9 +808,8 @@ extern "C" int mb200_embedding_fwd(const void* table, const int64_t* ids, void* 
   if (rows <= 0) return 0;
   if (d % 8) return 1001;
   const long long total = (long long)rows * (d / 8);
-  embedding_fwd_kernel<<<blocks_for(total, 256), 256, 0, ST(stream)>>>(CBF(table), ids, BF(out),
-                                                                       total, d);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(embedding_fwd_kernel, blocks_for(total, 256), 256, 0, ST(stream),
+                         CBF(table), ids, BF(out), total, d);
 }
 extern "C" int mb200_embedding_bwd(const void* dout, const int64_t* ids, void* dtable, int rows,
                                    int d, void* stream) {
@@ -817,20 +818,17 @@ extern "C" int mb200_embedding_bwd(const void* dout, const int64_t* ids, void* d
   if (d <= 0) return 0;
   if (d % 8 == 0 && aligned16(dout) && aligned16(dtable)) {
     const int nt = row_threads(d / 8);
-    embedding_bwd_vec_kernel<<<dim3(rows, blocks_for(d / 8, nt)), nt, 0, ST(stream)>>>(
-        CBF(dout), ids, BF(dtable), d);
-    return (int)cudaGetLastError();
+    return (int)launch_dep(embedding_bwd_vec_kernel, dim3(rows, blocks_for(d / 8, nt)), nt, 0,
+                           ST(stream), CBF(dout), ids, BF(dtable), d);
   }
   const long long total = (long long)rows * (d / 2);
-  embedding_bwd_kernel<<<blocks_for(total, 256), 256, 0, ST(stream)>>>(CBF(dout), ids, BF(dtable),
-                                                                       total, d);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(embedding_bwd_kernel, blocks_for(total, 256), 256, 0, ST(stream),
+                         CBF(dout), ids, BF(dtable), total, d);
 }
 
 extern "C" int mb200_sumsq(const void* x, int64_t n, int is_bf16, float* out, void* stream) {
   if (n <= 0) return 0;
-  sumsq_kernel<<<592, 256, 0, ST(stream)>>>(x, n, is_bf16, out);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(sumsq_kernel, 592, 256, 0, ST(stream), x, n, is_bf16, out);
 }
 
 // ------------------------------------------------- allocation-free RMSNorm backward ----

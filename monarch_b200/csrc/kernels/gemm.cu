@@ -74,8 +74,8 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  gemm_bf16_kernel<A_MN, B_MN, BN><<<grid, GEMM_THREADS, GemmTile<BN>::kSmemBytes, st>>>(ta, tb, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(gemm_bf16_kernel<A_MN, B_MN, BN>, grid, GEMM_THREADS,
+                         GemmTile<BN>::kSmemBytes, st, ta, tb, p);
 }
 
 static int make_gemm_tmaps_bn(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B,
@@ -172,6 +172,7 @@ __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   volatile int* abort_word = &sh->abort_word;
+  dep_wait();
 
   if (warp == 0) {
     if (elect_one()) {
@@ -318,9 +319,8 @@ template <bool A_MN, bool B_MN, int BN, int SPLIT>
 static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
                         int tiles, cudaStream_t st) {
   if (split_capacity<A_MN, B_MN, BN, SPLIT>() <= 0) return 1002;
-  gemm_split_kernel<A_MN, B_MN, BN, SPLIT>
-      <<<tiles * SPLIT, GEMM_THREADS, GemmTile<BN>::kSmemBytes, st>>>(ta, tb, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(gemm_split_kernel<A_MN, B_MN, BN, SPLIT>, tiles * SPLIT, GEMM_THREADS,
+                         GemmTile<BN>::kSmemBytes, st, ta, tb, p);
 }
 template <int BN, int SPLIT>
 static int launch_split_ab(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
@@ -386,8 +386,8 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParam
   if (cap <= 0) return 1002;
   const int tiles = ((p.M + G2_BM - 1) / G2_BM) * ((p.N + G2_BN - 1) / G2_BN);
   const int pairs = tiles < cap ? tiles : cap;
-  gemm2_bf16_kernel<A_MN, B_MN><<<2 * pairs, GEMM_THREADS, G2_SMEM_BYTES, st>>>(ta, tb, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dep(gemm2_bf16_kernel<A_MN, B_MN>, 2 * pairs, GEMM_THREADS, G2_SMEM_BYTES, st,
+                         ta, tb, p);
 }
 
 int make_gemm2_tmaps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B, int M, int N,

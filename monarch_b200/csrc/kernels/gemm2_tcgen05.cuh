@@ -80,12 +80,6 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
   const uint32_t cta = cluster_ctarank();  // 0: issues the MMAs; 1: partner
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int M = gemm_dyn_m(p);
-  const int Kd = gemm_dyn_k(p);
-  const int m_blocks = (M + G2_BM - 1) / G2_BM;
-  const int n_blocks = (p.N + G2_BN - 1) / G2_BN;
-  const int k_iters = (Kd + G2_BK - 1) / G2_BK;
-  const int num_tiles = m_blocks * n_blocks;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < G2_STAGES; ++s) {
@@ -109,6 +103,13 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   volatile int* abort_word = &sh->abort_word;
+  dep_wait();   // row counts and operands below come from kernels ahead in the stream
+  const int M = gemm_dyn_m(p);
+  const int Kd = gemm_dyn_k(p);
+  const int m_blocks = (M + G2_BM - 1) / G2_BM;
+  const int n_blocks = (p.N + G2_BN - 1) / G2_BN;
+  const int k_iters = (Kd + G2_BK - 1) / G2_BK;
+  const int num_tiles = m_blocks * n_blocks;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer

@@ -14,6 +14,7 @@
 //   move peer data; the TMA producer can be gated on global "ready" flags per block
 //   of B rows (bounded wait).
 #pragma once
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace mb200 {
@@ -258,12 +259,6 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int M = gemm_dyn_m(p);
-  const int Kd = gemm_dyn_k(p);
-  const int m_blocks = (M + GEMM_BM - 1) / GEMM_BM;
-  const int n_blocks = (p.N + BN - 1) / BN;
-  const int k_iters = (Kd + GEMM_BK - 1) / GEMM_BK;
-  const int num_tiles = m_blocks * n_blocks;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -286,6 +281,13 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   volatile int* abort_word = &sh->abort_word;
+  dep_wait();   // row counts and operands below come from kernels ahead in the stream
+  const int M = gemm_dyn_m(p);
+  const int Kd = gemm_dyn_k(p);
+  const int m_blocks = (M + GEMM_BM - 1) / GEMM_BM;
+  const int n_blocks = (p.N + BN - 1) / BN;
+  const int k_iters = (Kd + GEMM_BK - 1) / GEMM_BK;
+  const int num_tiles = m_blocks * n_blocks;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
