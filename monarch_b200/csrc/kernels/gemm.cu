@@ -55,26 +55,26 @@ int sm_count() {
   return n;
 }
 
-template <bool A_MN, bool B_MN, int BN>
+template <bool A_MN, bool B_MN, int BN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA,
                      const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_cta_body<A_MN, B_MN, BN>(&tmA, &tmB, p, blockIdx.x, gridDim.x, smem_raw);
+  gemm_cta_body<A_MN, B_MN, BN, EPI>(&tmA, &tmB, p, blockIdx.x, gridDim.x, smem_raw);
 }
 
-template <bool A_MN, bool B_MN, int BN>
+template <bool A_MN, bool B_MN, int BN, int EPI = kEpiStore>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
                   cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, BN>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          GemmTile<BN>::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return (int)launch_dep(gemm_bf16_kernel<A_MN, B_MN, BN>, grid, GEMM_THREADS,
+  return (int)launch_dep(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>, grid, GEMM_THREADS,
                          GemmTile<BN>::kSmemBytes, st, ta, tb, p);
 }
 
@@ -339,27 +339,27 @@ static int launch_split_n(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
 }
 
 // ------------------------------------------------------------------ CTA-pair variant
-template <bool A_MN, bool B_MN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+template <bool A_MN, bool B_MN, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm2_threads(EPI), 1)
     gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  gemm2_cta_body<A_MN, B_MN>(&tmA, &tmB, p, blockIdx.x >> 1, gridDim.x >> 1, smem_raw);
+  gemm2_cta_body<A_MN, B_MN, EPI>(&tmA, &tmB, p, blockIdx.x >> 1, gridDim.x >> 1, smem_raw);
 }
 
 // Number of CTA pairs that can be resident at once (<= SMs / 2; fewer when a GPC has an
 // odd number of usable SMs).  Queried once per operand-layout variant.
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI>
 static int pair_capacity() {
   static int cap = 0;
   if (cap) return cap;
-  if (cudaFuncSetAttribute(gemm2_bf16_kernel<A_MN, B_MN>,
+  if (cudaFuncSetAttribute(gemm2_bf16_kernel<A_MN, B_MN, EPI>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
                            G2_SMEM_BYTES) != cudaSuccess)
     return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (sm_count() / 2));
-  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.blockDim = dim3(gemm2_threads(EPI));
   cfg.dynamicSmemBytes = G2_SMEM_BYTES;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -369,7 +369,7 @@ static int pair_capacity() {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<A_MN, B_MN>, &cfg) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<A_MN, B_MN, EPI>, &cfg) != cudaSuccess ||
       n <= 0) {
     cudaGetLastError();
     n = sm_count() / 2;
@@ -379,15 +379,15 @@ static int pair_capacity() {
   return cap;
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI = kEpiStore>
 static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
                    cudaStream_t st) {
-  const int cap = pair_capacity<A_MN, B_MN>();
+  const int cap = pair_capacity<A_MN, B_MN, EPI>();
   if (cap <= 0) return 1002;
   const int tiles = ((p.M + G2_BM - 1) / G2_BM) * ((p.N + G2_BN - 1) / G2_BN);
   const int pairs = tiles < cap ? tiles : cap;
-  return (int)launch_dep(gemm2_bf16_kernel<A_MN, B_MN>, 2 * pairs, GEMM_THREADS, G2_SMEM_BYTES, st,
-                         ta, tb, p);
+  return (int)launch_dep(gemm2_bf16_kernel<A_MN, B_MN, EPI>, 2 * pairs, gemm2_threads(EPI),
+                         G2_SMEM_BYTES, st, ta, tb, p);
 }
 
 int make_gemm2_tmaps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B, int M, int N,
@@ -496,6 +496,100 @@ extern "C" int mb200_gemm_bf16(const void* A, const void* B, void* C, const void
   if (bn == 64) return launch_gemm_bn<64>(ta, tb, p, a_mn, b_mn, grid, st);
   if (bn == 128) return launch_gemm_bn<128>(ta, tb, p, a_mn, b_mn, grid, st);
   return launch_gemm(ta, tb, p, a_mn, b_mn, grid, st);
+}
+
+// ------------------------------------------------------- gated activation in the epilogue
+// C[M, F] = silu(A Wg^T) * (A Wu^T) with W = [Wg; Wu] of 2F rows; gu ([M, 2F], or null) gets the
+// two products.  The gate and up columns of an output column meet in one tile because its B rows
+// come from both halves of W.
+//
+// What it saves is the pass over memory (and for small products the launch); what it costs is a
+// longer epilogue, which the next tile's products hide if K is long enough.  Product plus
+// activation as two kernels -> as one, us, the two timed in turn:
+//   forward without gu   T 8192 F 14336 K 4096 1528 -> 1351, K 2048 F 8192 503 -> 409,
+//                        K 1024 F 4096 200 -> 164, K 512 F 8192 349 -> 296
+//   forward with gu      T 8192 F 14336 K 4096 1528 -> 1393, K 2560 F 4096 256 -> 245,
+//                        K 2048 F 8192 503 -> 540 (two kernels there)
+//   backward             T 8192 F 14336 K 4096 978 -> 855, K 3072 F 8192 454 -> 433,
+//                        K 2560 F 4096 189 -> 197 (two kernels there)
+//   256x512x256 on small tiles 22.0 -> 14.7 and 21.5 -> 13.9 with the host's part.
+constexpr int kGluFwdMinK = 0, kGluFwdKeepMinK = 2560, kGluBwdMinK = 3072;
+
+// 1: CTA-pair tile, 0: small single-CTA tile, -1: two kernels are faster (or only they can).
+static int glu_tile(int M, int N, int F, int K, int min_k, GemmPlan* plan) {
+  *plan = g_gemm_impl == 2 ? gemm_plan(M, N, K) : GemmPlan{128, 1};
+  if (plan->split > 1) return -1;
+  if (plan->bn != 0 && plan->bn != 256) return 0;
+  return F % 128 == 0 && K >= min_k ? 1 : -1;
+}
+
+extern "C" int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void* gu, int M, int F,
+                                     int K, int lda, int ldw, int ldh, int ld_gu, int* status,
+                                     void* stream) {
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  if (F % 64 || (ldh & 7) || (ld_gu & 7) || ((reinterpret_cast<uintptr_t>(H) |
+                                              reinterpret_cast<uintptr_t>(gu)) & 15))
+    return 1001;
+  GemmPlan plan;
+  const int tile = glu_tile(M, 2 * F, F, K, gu ? kGluFwdKeepMinK : kGluFwdMinK, &plan);
+  if (tile < 0) return MB200_NOT_FUSED;
+  GemmParams p{};
+  p.C = reinterpret_cast<__nv_bfloat16*>(H);
+  p.M = M; p.N = 2 * F; p.K = K;
+  p.ldc = ldh;
+  p.status = status;
+  p.flag_chunk_elems = 1;
+  p.gu_out = reinterpret_cast<__nv_bfloat16*>(gu);
+  p.ld_gu = ld_gu;
+  p.glu_f = F;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  CUtensorMap ta, tb;
+  if (tile == 1) {
+    const int r = make_gemm2_tmaps(&ta, &tb, A, W, M, 2 * F, K, lda, ldw, 0, 0);
+    if (r) return 1000 - r;
+    return gu ? launch2<false, false, kEpiSwigluFwdKeep>(ta, tb, p, st)
+              : launch2<false, false, kEpiSwigluFwd>(ta, tb, p, st);
+  }
+  const int r = make_gemm_tmaps_bn(&ta, &tb, A, W, M, 2 * F, K, lda, ldw, 0, 0, 64);
+  if (r) return 1000 - r;
+  const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * (F / 64);
+  const int grid = tiles < sm_count() ? tiles : sm_count();
+  return gu ? launch<false, false, 128, kEpiSwigluFwdKeep>(ta, tb, p, grid, st)
+            : launch<false, false, 128, kEpiSwigluFwd>(ta, tb, p, grid, st);
+}
+
+// dgu[M, 2F] = gradient of silu(gate) * up at gu for dh = A W (W [K, F] row-major), without
+// storing dh.
+extern "C" int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* gu, void* dgu, int M,
+                                     int F, int K, int lda, int ldw, int ld_gu, int* status,
+                                     void* stream) {
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  if (F % 32 || (ld_gu & 7) || ((reinterpret_cast<uintptr_t>(gu) |
+                                 reinterpret_cast<uintptr_t>(dgu)) & 15))
+    return 1001;
+  GemmPlan plan;
+  const int tile = glu_tile(M, F, F, K, kGluBwdMinK, &plan);
+  if (tile < 0) return MB200_NOT_FUSED;
+  GemmParams p{};
+  p.M = M; p.N = F; p.K = K;
+  p.status = status;
+  p.flag_chunk_elems = 1;
+  p.gu_in = reinterpret_cast<const __nv_bfloat16*>(gu);
+  p.gu_out = reinterpret_cast<__nv_bfloat16*>(dgu);
+  p.ld_gu = ld_gu;
+  p.glu_f = F;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  CUtensorMap ta, tb;
+  if (tile == 1) {
+    const int r = make_gemm2_tmaps(&ta, &tb, A, W, M, F, K, lda, ldw, 0, 1);
+    return r ? 1000 - r : launch2<false, true, kEpiSwigluBwd>(ta, tb, p, st);
+  }
+  const int r = make_gemm_tmaps_bn(&ta, &tb, A, W, M, F, K, lda, ldw, 0, 1, plan.bn);
+  if (r) return 1000 - r;
+  const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((F + plan.bn - 1) / plan.bn);
+  const int grid = tiles < sm_count() ? tiles : sm_count();
+  return plan.bn == 64 ? launch<false, true, 64, kEpiSwigluBwd>(ta, tb, p, grid, st)
+                       : launch<false, true, 128, kEpiSwigluBwd>(ta, tb, p, grid, st);
 }
 
 extern "C" int mb200_gemm_set_impl(int impl) {

@@ -69,7 +69,15 @@ struct Gemm2Shared {
   volatile int abort_word;
 };
 
-template <bool A_MN, bool B_MN>
+// Threads of a CTA.  Two of the gated epilogues have more to read or compute per tile and take
+// eight warps, two per TMEM lane quadrant, each with half of the columns; the one that also
+// stores gate and up is slower with eight (K 4096, T 4096: 744 us against 681).
+__host__ __device__ constexpr int gemm2_epi_warps(int epi) {
+  return epi == kEpiSwigluFwd || epi == kEpiSwigluBwd ? 8 : 4;
+}
+__host__ __device__ constexpr int gemm2_threads(int epi) { return 64 + 32 * gemm2_epi_warps(epi); }
+
+template <bool A_MN, bool B_MN, int EPI = kEpiStore>
 __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUtensorMap* tmB,
                                                const GemmParams& p, int vpair, int npairs,
                                                uint8_t* smem_raw) {
@@ -88,7 +96,7 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&sh->tmem_full[s], 1);
-      mbar_init(&sh->tmem_empty[s], 8);
+      mbar_init(&sh->tmem_empty[s], 2 * gemm2_epi_warps(EPI));
     }
     sh->abort_word = 0;
     mbar_fence_init();
@@ -124,7 +132,9 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
         tile_coords(t, m_blocks, n_blocks, p.n_blk_rot, p.b_ready != nullptr, p.m_group, p.m_rot,
                     m_blk, n_blk);
         const int m0 = m_blk * G2_BM + (int)cta * G2_HALF;
-        const int n0 = n_blk * G2_BN + (int)cta * G2_HALF;
+        // gated forward: the even CTA stages gate rows, the odd one the same up columns' rows
+        const int n0 = epi_swiglu_fwd(EPI) ? n_blk * G2_HALF + (cta ? p.glu_f : 0)
+                                           : n_blk * G2_BN + (int)cta * G2_HALF;
         bool ok = true;
         if (p.b_ready && n0 < p.N) {
           int last = n0 + G2_HALF - 1;
@@ -221,6 +231,7 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
   } else {
     // ---------------------------------------------------------------- epilogue
     const int quad = warp & 3;
+    const int part = (warp - 2) >> 2;   // which half of the columns (gated epilogues)
     int acc = 0;
     uint32_t acc_phase = 0;
     const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
@@ -233,19 +244,46 @@ __device__ __forceinline__ void gemm2_cta_body(const CUtensorMap* tmA, const CUt
                     m_blk, n_blk);
       const int row = m_blk * G2_BM + (int)cta * G2_HALF + quad * 32 + lane;
       const int n0 = n_blk * G2_BN;
+      constexpr int kHalfCols = G2_BN / 2;
+      const int c0 = n0 + part * kHalfCols;
+      GluStrip ahead;   // of the next strip; the first one's loads run under the wait
+      if constexpr (EPI == kEpiSwigluBwd) glu_load(p, ahead, row, c0, M);
       if (!mbar_wait(&sh->tmem_full[acc], acc_phase, abort_word, p.status)) break;
       tc_fence_after();
       const uint32_t t_base = tmem_base + acc * G2_BN + ((uint32_t)(quad * 32) << 16);
+      if constexpr (epi_swiglu_fwd(EPI)) {
+        constexpr int kStrips = G2_HALF / 32 / (gemm2_epi_warps(EPI) / 4);   // per warp
 #pragma unroll 1
-      for (int c = 0; c < G2_BN / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(t_base + c * 32, v);
-        tmem_ld_wait();
-        if (k_iters == 0) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = 0u;
+        for (int c = part * kStrips; c < (part + 1) * kStrips; ++c) {
+          uint32_t vg[32], vu[32];
+          tmem_ld_32x32b_x32(t_base + c * 32, vg);
+          tmem_ld_32x32b_x32(t_base + G2_HALF + c * 32, vu);
+          tmem_ld_wait();
+          gemm_store_swiglu_fwd<EPI == kEpiSwigluFwdKeep>(p, vg, vu, row,
+                                                          n_blk * G2_HALF + c * 32, M);
         }
-        gemm_store_strip(p, v, row, n0 + c * 32, vec_ok, M);
+      } else if constexpr (EPI == kEpiSwigluBwd) {
+#pragma unroll 1
+        for (int c = 0; c < kHalfCols / 32; ++c) {
+          const GluStrip now = ahead;
+          if (c + 1 < kHalfCols / 32) glu_load(p, ahead, row, c0 + (c + 1) * 32, M);
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(t_base + part * kHalfCols + c * 32, v);
+          tmem_ld_wait();
+          gemm_store_swiglu_bwd(p, v, now, row, c0 + c * 32, M);
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < G2_BN / 32; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(t_base + c * 32, v);
+          tmem_ld_wait();
+          if (k_iters == 0) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0u;
+          }
+          gemm_store_strip(p, v, row, n0 + c * 32, vec_ok, M);
+        }
       }
       tc_fence_before();
       __syncwarp();

@@ -85,7 +85,94 @@ struct GemmParams {
   const int* sc_slot;
   void* sc_out[8];
   int sc_ld;
+  // Gated-activation epilogues (kEpiSwiglu*): gu and dgu are [M, 2F] with
+  // leading dimension ld_gu, gate columns first, F = glu_f.
+  const __nv_bfloat16* gu_in;
+  __nv_bfloat16* gu_out;
+  int ld_gu;
+  int glu_f;
 };
+
+// What the epilogue makes of a finished tile.
+enum : int {
+  kEpiStore = 0,      // C (+ R) (+ C), or one of the reduce-scatter / scatter stores
+  kEpiSwigluFwd = 1,      // B = [gate rows; up rows] of 2F: C[M, F] = silu(gate) * up
+  kEpiSwigluFwdKeep = 2,  // the same, and gu_out = the two products
+  kEpiSwigluBwd = 3,      // result = dh[M, F]: gu_out = d(gate), d(up) from gu_in; dh is not stored
+};
+__host__ __device__ constexpr bool epi_swiglu_fwd(int epi) {
+  return epi == kEpiSwigluFwd || epi == kEpiSwigluFwdKeep;
+}
+
+// Both gated epilogues work on values rounded to bf16 first, like the separate kernels that
+// read them from memory: the results have the same bits.
+__device__ __forceinline__ float bf16_round(uint32_t fp32_bits) {
+  return __bfloat162float(__float2bfloat16(__uint_as_float(fp32_bits)));
+}
+// 32 columns of gate and up accumulators of one row.  Requires glu_f % 32 == 0 and 16-byte
+// aligned rows (checked by the caller).
+template <bool KEEP>
+__device__ __forceinline__ void gemm_store_swiglu_fwd(const GemmParams& p, const uint32_t (&vg)[32],
+                                                      const uint32_t (&vu)[32], int row, int col,
+                                                      int M) {
+  if (row >= M || col >= p.glu_f) return;
+  __nv_bfloat16* hp = p.C + (size_t)row * p.ldc + col;
+  __nv_bfloat16* gp = KEEP ? p.gu_out + (size_t)row * p.ld_gu + col : nullptr;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t h[4], g4[4], u4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = q * 8 + i * 2;
+      const float g0 = bf16_round(vg[e]), g1 = bf16_round(vg[e + 1]);
+      const float u0 = bf16_round(vu[e]), u1 = bf16_round(vu[e + 1]);
+      h[i] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
+      g4[i] = pack_bf16x2(g0, g1);
+      u4[i] = pack_bf16x2(u0, u1);
+    }
+    *reinterpret_cast<uint4*>(hp + q * 8) = make_uint4(h[0], h[1], h[2], h[3]);
+    if (KEEP) {
+      *reinterpret_cast<uint4*>(gp + q * 8) = make_uint4(g4[0], g4[1], g4[2], g4[3]);
+      *reinterpret_cast<uint4*>(gp + p.glu_f + q * 8) = make_uint4(u4[0], u4[1], u4[2], u4[3]);
+    }
+  }
+}
+// gate and up of 32 columns of one row, loaded ahead of the accumulators they meet
+struct GluStrip {
+  uint4 g[4], u[4];
+};
+__device__ __forceinline__ void glu_load(const GemmParams& p, GluStrip& s, int row, int col,
+                                         int M) {
+  if (row >= M || col >= p.glu_f) return;
+  const __nv_bfloat16* gp = p.gu_in + (size_t)row * p.ld_gu + col;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    s.g[q] = *reinterpret_cast<const uint4*>(gp + q * 8);
+    s.u[q] = *reinterpret_cast<const uint4*>(gp + p.glu_f + q * 8);
+  }
+}
+__device__ __forceinline__ void gemm_store_swiglu_bwd(const GemmParams& p, const uint32_t (&v)[32],
+                                                      const GluStrip& s, int row, int col, int M) {
+  if (row >= M || col >= p.glu_f) return;
+  __nv_bfloat16* dp = p.gu_out + (size_t)row * p.ld_gu + col;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t gw[4] = {s.g[q].x, s.g[q].y, s.g[q].z, s.g[q].w};
+    const uint32_t uw[4] = {s.u[q].x, s.u[q].y, s.u[q].z, s.u[q].w};
+    uint32_t dg[4], du[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 g = unpack_bf16x2(gw[i]), u = unpack_bf16x2(uw[i]);
+      const float d0 = bf16_round(v[q * 8 + i * 2]), d1 = bf16_round(v[q * 8 + i * 2 + 1]);
+      const float s0 = 1.f / (1.f + __expf(-g.x)), s1 = 1.f / (1.f + __expf(-g.y));
+      du[i] = pack_bf16x2(d0 * (g.x * s0), d1 * (g.y * s1));
+      dg[i] = pack_bf16x2(d0 * u.x * s0 * (1.f + g.x * (1.f - s0)),
+                          d1 * u.y * s1 * (1.f + g.y * (1.f - s1)));
+    }
+    *reinterpret_cast<uint4*>(dp + q * 8) = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+    *reinterpret_cast<uint4*>(dp + p.glu_f + q * 8) = make_uint4(du[0], du[1], du[2], du[3]);
+  }
+}
 
 __device__ __forceinline__ int gemm_dyn_m(const GemmParams& p) {
   if (p.dyn_m_nparts <= 0) return p.M;
@@ -246,7 +333,7 @@ struct GemmShared {
   volatile int abort_word;
 };
 
-template <bool A_MN, bool B_MN, int BN = GEMM_BN>
+template <bool A_MN, bool B_MN, int BN = GEMM_BN, int EPI = kEpiStore>
 __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUtensorMap* tmB,
                                               const GemmParams& p, int vcta, int nvcta,
                                               uint8_t* smem_raw) {
@@ -340,6 +427,10 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(sb + j * 8192, tmB, &sh->full[stage], n0 + j * 64, k0);
+          } else if (epi_swiglu_fwd(EPI)) {   // half the rows are gate, half the same up columns
+            const int f0 = n_blk * (BN / 2);
+            tma_load_2d(sb, tmB, &sh->full[stage], k0, f0);
+            tma_load_2d(sb + BN / 2 * 128, tmB, &sh->full[stage], k0, p.glu_f + f0);
           } else {
             tma_load_2d(sb, tmB, &sh->full[stage], k0, n0);
           }
@@ -408,19 +499,43 @@ __device__ __forceinline__ void gemm_cta_body(const CUtensorMap* tmA, const CUte
       if (n_blk >= n_blocks) n_blk -= n_blocks;
       const int row = m_blk * GEMM_BM + quad * 32 + lane;
       const int n0 = n_blk * BN;
+      GluStrip ahead;   // of the next strip; the first one's loads run under the wait
+      if constexpr (EPI == kEpiSwigluBwd) glu_load(p, ahead, row, n0, M);
       if (!mbar_wait(&sh->tmem_full[acc], acc_phase, abort_word, p.status)) break;
       tc_fence_after();
       const uint32_t t_base = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16);
+      if constexpr (epi_swiglu_fwd(EPI)) {
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(t_base + c * 32, v);
-        tmem_ld_wait();
-        if (k_iters == 0) {  // empty reduction (no tokens): the accumulator was never written
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = 0u;
+        for (int c = 0; c < BN / 64; ++c) {
+          uint32_t vg[32], vu[32];
+          tmem_ld_32x32b_x32(t_base + c * 32, vg);
+          tmem_ld_32x32b_x32(t_base + BN / 2 + c * 32, vu);
+          tmem_ld_wait();
+          gemm_store_swiglu_fwd<EPI == kEpiSwigluFwdKeep>(p, vg, vu, row, n_blk * (BN / 2) + c * 32,
+                                                          M);
         }
-        gemm_store_strip(p, v, row, n0 + c * 32, vec_ok, M);
+      } else if constexpr (EPI == kEpiSwigluBwd) {
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          const GluStrip now = ahead;
+          if (c + 1 < BN / 32) glu_load(p, ahead, row, n0 + (c + 1) * 32, M);
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(t_base + c * 32, v);
+          tmem_ld_wait();
+          gemm_store_swiglu_bwd(p, v, now, row, n0 + c * 32, M);
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(t_base + c * 32, v);
+          tmem_ld_wait();
+          if (k_iters == 0) {  // empty reduction (no tokens): the accumulator was never written
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0u;
+          }
+          gemm_store_strip(p, v, row, n0 + c * 32, vec_ok, M);
+        }
       }
       tc_fence_before();
       __syncwarp();

@@ -14,8 +14,18 @@ int mb200_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M,
                     int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int accumulate,
                     int* status, void* stream);
 
+// H[M,F] = silu(A Wg^T) * (A Wu^T), W = [Wg; Wu] row-major [2F,K]; gu ([M,2F], may be null)
+// receives the two products.  F % 64 == 0.  Both functions return MB200_NOT_FUSED, and launch
+// nothing, for products that are faster as two kernels.
+#define MB200_NOT_FUSED 1003
+int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void* gu, int M, int F, int K,
+                          int lda, int ldw, int ldh, int ld_gu, int* status, void* stream);
+// dgu[M,2F] = gradient of silu(gate)*up at gu for dh = A W, W row-major [K,F].  F % 32 == 0.
+int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* gu, void* dgu, int M, int F,
+                          int K, int lda, int ldw, int ld_gu, int* status, void* stream);
+
 // Which GEMM kernel the library uses: 1 = single-CTA 128x256 tiles, 2 = CTA-pair 256x256
-// tiles (default).  The fused collective+GEMM kernels follow the same setting.
+// tiles, or smaller ones for products with few tiles (default).  The fused collective+GEMM kernels follow the same setting.
 int mb200_gemm_set_impl(int impl);
 int mb200_gemm_get_impl(void);
 

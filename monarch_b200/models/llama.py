@@ -393,8 +393,11 @@ class LlamaEngine:
         """x2 -> x2 + mlp(norm(x2)); without ``need_out`` only what the backward reads (the
         down projection's result is no part of it) and None in its place."""
         h2, rstd2 = ops.rmsnorm_fwd(x2, w["mlp_norm"], self.cfg.eps)
-        gu = _unit_gemm(w, h2, "w_gu")
-        hmid = ops.swiglu_fwd(gu)
+        if hasattr(w, "gemm"):    # weights that arrive inside the product (see _unit_gemm)
+            gu = _unit_gemm(w, h2, "w_gu")
+            hmid = ops.swiglu_fwd(gu)
+        else:
+            hmid, gu = ops.gemm_swiglu(h2, w["w_gu"], keep_gu=keep)
         y = ops.gemm(hmid, w["w_down"], residual=x2) if need_out else None
         return y, ((x2, rstd2, h2, gu, hmid) if keep else None)
 
@@ -412,10 +415,8 @@ class LlamaEngine:
     def _mlp_bwd(self, w: dict, g: dict, sm, dy: torch.Tensor):
         """Gradient w.r.t. x2 (residual path included)."""
         x2, rstd2, h2, gu, hmid = sm
-        d_hmid = ops.gemm(dy, w["w_down"], b_mn=True)
+        d_gu = ops.gemm_swiglu_bwd(dy, w["w_down"], gu)
         ops.gemm(dy, hmid, a_mn=True, b_mn=True, out=g["w_down"])
-        d_gu = ops.swiglu_bwd(gu, d_hmid)
-        del d_hmid
         d_h2 = ops.gemm(d_gu, w["w_gu"], b_mn=True)
         ops.gemm(d_gu, h2, a_mn=True, b_mn=True, out=g["w_gu"])
         del d_gu

@@ -131,11 +131,12 @@ def rope_(qkv, cos, sin, seq_len, n_rot_heads, hd, inverse=False):
     return qkv
 
 
-def swiglu_fwd(gu):
+def swiglu_fwd(gu, out=None):
     rows, F2 = gu.shape
     if not gu.is_cuda:
-        return R.swiglu_fwd(gu).to(gu.dtype)
-    h = torch.empty(rows, F2 // 2, dtype=gu.dtype, device=gu.device)
+        h = R.swiglu_fwd(gu).to(gu.dtype)
+        return h if out is None else out.copy_(h)
+    h = torch.empty(rows, F2 // 2, dtype=gu.dtype, device=gu.device) if out is None else out
     K.check(K.lib().mb200_swiglu_fwd(gu.data_ptr(), h.data_ptr(), rows, F2 // 2, K.stream_ptr()),
             "swiglu_fwd")
     return h
@@ -153,6 +154,54 @@ def swiglu_bwd(gu, dh, out=None):
     K.check(K.lib().mb200_swiglu_bwd(gu.data_ptr(), dh.data_ptr(), dgu.data_ptr(), rows, F2 // 2,
                                      K.stream_ptr()), "swiglu_bwd")
     return dgu
+
+
+_NOT_FUSED = 1003   # MB200_NOT_FUSED: this product is faster as two kernels
+
+
+def gemm_swiglu(a, w_gu, keep_gu=True):
+    """``gu = a @ w_gu.T`` ([rows, 2F]) and ``h = swiglu_fwd(gu)``; returns (h, gu), without
+    ``keep_gu`` (h, None).  One kernel where that is faster, with the bits of the two."""
+    T, F = a.shape[0], w_gu.shape[0] // 2
+    if a.is_cuda and T and not F % 64 and a.dtype == bf16 and w_gu.dtype == bf16:
+        a, lda = _rowmajor(a)
+        w_gu, ldw = _rowmajor(w_gu)
+        Kd = a.shape[1]
+        assert w_gu.shape == (2 * F, Kd), (a.shape, w_gu.shape)
+        h = torch.empty(T, F, dtype=bf16, device=a.device)
+        gu = torch.empty(T, 2 * F, dtype=bf16, device=a.device) if keep_gu else None
+        rc = K.lib().mb200_gemm_swiglu_fwd(
+            a.data_ptr(), w_gu.data_ptr(), h.data_ptr(), _p(gu), T, F, Kd, lda, ldw, F, 2 * F,
+            K.status_ptr(a), K.stream_ptr())
+        if rc != _NOT_FUSED:
+            K.check(rc, "gemm_swiglu_fwd")
+            return h, gu
+        if keep_gu:
+            return swiglu_fwd(gemm(a, w_gu, out=gu), out=h), gu
+        return swiglu_fwd(gemm(a, w_gu), out=h), None
+    gu = gemm(a, w_gu)
+    return swiglu_fwd(gu), (gu if keep_gu else None)
+
+
+def gemm_swiglu_bwd(dy, w_down, gu):
+    """``swiglu_bwd(gu, dy @ w_down)``; one kernel where that is faster, with the bits of the
+    two."""
+    T, F = dy.shape[0], w_down.shape[1]
+    if (dy.is_cuda and T and not F % 32 and dy.dtype == bf16 and w_down.dtype == bf16
+            and gu.dtype == bf16 and gu.is_contiguous() and not gu.data_ptr() & 15):
+        dy, lda = _rowmajor(dy)
+        w_down, ldw = _rowmajor(w_down)
+        Kd = dy.shape[1]
+        assert w_down.shape[0] == Kd and gu.shape == (T, 2 * F), (dy.shape, w_down.shape, gu.shape)
+        dgu = torch.empty_like(gu)
+        rc = K.lib().mb200_gemm_swiglu_bwd(
+            dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, F, Kd, lda, ldw,
+            2 * F, K.status_ptr(dy), K.stream_ptr())
+        if rc != _NOT_FUSED:
+            K.check(rc, "gemm_swiglu_bwd")
+            return dgu
+        return swiglu_bwd(gu, gemm(dy, w_down, b_mn=True), out=dgu)
+    return swiglu_bwd(gu, gemm(dy, w_down, b_mn=True))
 
 
 def cross_entropy_(logits, targets, grad_scale):
