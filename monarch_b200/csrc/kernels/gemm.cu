@@ -430,6 +430,16 @@ struct GemmPlan {
   int bn;      // 0: the CTA pair's 256x256 tile, else the columns of a single CTA's 128-row tile
   int split;   // CTAs of a cluster that share a tile along K
 };
+// Clusters of `split` CTAs that run at once (they have to share a GPC: fewer than SMs / split).
+static int split_clusters(int bn, int split) {
+  if (bn == 64)
+    return split == 2   ? split_capacity<false, false, 64, 2>()
+           : split == 4 ? split_capacity<false, false, 64, 4>()
+                        : split_capacity<false, false, 64, 8>();
+  return split == 2   ? split_capacity<false, false, 128, 2>()
+         : split == 4 ? split_capacity<false, false, 128, 4>()
+                      : split_capacity<false, false, 128, 8>();
+}
 static GemmPlan gemm_plan(int M, int N, int K) {
   const int iters = (K + GEMM_BK - 1) / GEMM_BK;
   const auto div = [](long long a, long long b) { return (a + b - 1) / b; };
@@ -448,8 +458,8 @@ static GemmPlan gemm_plan(int M, int N, int K) {
     if (k.bn == 256) continue;
     for (int i = 0; i < 3; ++i) {
       const int split = 2 << i;
-      // one wave only: clusters of 8 fill 16 of every GPC's 18 to 20 SMs
-      if (tiles * split > (split == 2 ? sms - 4 : sms * 7 / 8) || iters < 2 * split) break;
+      // one wave only
+      if (tiles * split > sms || iters < 2 * split || tiles > split_clusters(k.bn, split)) break;
       const float v = k.t0 + k.t_split[i] + k.c * div(iters, split);
       if (v < t) t = v, best = {k.bn, split};
     }
