@@ -6,8 +6,8 @@
 //      shared memory, walks over every query block at or below the diagonal of every
 //      query head of the group, and accumulates dV += P^T dO and dK += dS^T Q in TMEM:
 //        S^T = K Q^T, dP^T = V dO^T      (tcgen05.mma, operands in shared memory)
-//        P^T = exp2(S^T c - lse), dS^T = P^T (dP^T - delta)   (8 warps, one kv row per
-//                                         thread, written back as bf16 over S^T / dP^T)
+//        P^T = exp2(S^T c - lse), dS^T = P^T (dP^T - delta)   (16 warps, a quarter of a
+//                                         kv row per thread, written back as bf16)
 //        dV += P^T dO, dK += dS^T Q      (A operand from TMEM, dO / Q MN-major from smem)
 //   3. dQ: one CTA per (query block, query head, batch), walks over the kv blocks up to
 //      the diagonal:  S = Q K^T, dP = dO V^T, dS = P (dP - delta), dQ += dS K.
