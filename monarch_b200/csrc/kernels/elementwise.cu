@@ -202,7 +202,12 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
     const int st = it % stages;
     const float rs = rs_next;
     if (it + 1 < n) rs_next = rstd[row + gridDim.x];
-    if (!mbar_wait(&full[st], (uint32_t)(it / stages) & 1, &abort_word, nullptr)) break;
+    if (!mbar_wait(&full[st], (uint32_t)(it / stages) & 1, &abort_word, nullptr)) {
+      // no status word here: a copy that never landed shows as NaN in the weight gradient
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) acc[ch][0] = __int_as_float(0x7fffffff);
+      break;
+    }
     const __nv_bfloat16* sx = reinterpret_cast<const __nv_bfloat16*>(
         ring + (size_t)st * NIN * row_bytes);
     float xh[NCH][8], g[NCH][8];

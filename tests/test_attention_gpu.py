@@ -147,3 +147,23 @@ def test_attention_backward_with_an_output_that_is_not_16_byte_aligned(hd):
     do2 = torch.empty(B * S, Hq * hd + 8, dtype=bf16, device="cuda")[:, :Hq * hd]
     do2.copy_(do)
     assert torch.equal(ops.attention_bwd(ctx2, do2), want)
+
+
+# one query block, an odd number of them (the second slot of the last pair is empty), groups of an
+# odd size (slots are row blocks, not heads), several batches
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(2, 128, 1, 1), (1, 384, 3, 3), (3, 640, 6, 2),
+                                        (1, 896, 8, 1)])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_blocks_and_groups(B, S, Hq, Hkv, hd):
+    from monarch_b200 import ops
+    torch.manual_seed(5)
+    T = B * S
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * hd, device="cuda").to(bf16)
+    do = torch.randn(T, Hq * hd, device="cuda").to(bf16)
+    o, ctx = ops.attention_fwd(qkv, B, S, Hq, Hkv, hd)
+    got = ops.attention_bwd(ctx, do)
+    o_ref, lse_ref, q, k, v = _reference(qkv, B, S, Hq, Hkv, hd, hd ** -0.5)
+    assert _rel(o, o_ref) < 5e-3 and (ctx.lse - lse_ref).abs().max().item() < 1e-3
+    g = [t.transpose(1, 2).reshape(T, -1)
+         for t in torch.autograd.grad(o_ref, (q, k, v), do.float())]
+    assert _rel(got, torch.cat(g, dim=1)) < 1e-2
