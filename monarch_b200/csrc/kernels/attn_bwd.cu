@@ -141,7 +141,9 @@ struct DkvBars {
   uint64_t q_full[AB_ST3], q_empty[AB_ST3];
   uint64_t do_full[AB_ST2], do_empty[AB_ST2];
   uint64_t ld_full[AB_ST2], ld_empty[AB_ST2];
-  uint64_t s_full, s_free, dp_full, p_half, p_ready, ds_ready, acc_done;
+  // P of step t signals p_half/p_ready[t & 1]: at hd 64 S(t+1) is issued ahead of the waits for
+  // P(t), so the warps may have handed over P(t+1) too before the issuing warp looks
+  uint64_t s_full, s_free, dp_full, p_half[2], p_ready[2], ds_ready, acc_done;
   uint32_t tmem_base;
   volatile int abort_word;
 };
@@ -235,8 +237,10 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->s_free, 16);
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->p_half, 16);
-    mbar_init(&bars->p_ready, 16);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&bars->p_half[s], 16);
+      mbar_init(&bars->p_ready[s], 16);
+    }
     mbar_init(&bars->ds_ready, 16);
     mbar_init(&bars->acc_done, 1);
     bars->abort_word = 0;
@@ -326,12 +330,13 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
           ok = mbar_wait(&bars->s_free, par, abort_word, p.status) && next_s(t);
           if (!ok) break;
         }
-        ok = mbar_wait(&bars->p_half, par, abort_word, p.status);
+        const uint32_t p_par = (uint32_t)(t >> 1) & 1;
+        ok = mbar_wait(&bars->p_half[t & 1], p_par, abort_word, p.status);
         if (!ok) break;
         tc_fence_after();
         const uint32_t tp = tmem_base + kColP + (kOwnP ? (t & 1) * 64 : 0);
         mma_grad_half<HD, kQuarterP>(tmem_base + kColDV, tp, sdo + d2 * SM::kTile, 0, t > 0);
-        ok = mbar_wait(&bars->p_ready, par, abort_word, p.status);
+        ok = mbar_wait(&bars->p_ready[t & 1], p_par, abort_word, p.status);
         if (!ok) break;
         tc_fence_after();
         mma_grad_half<HD, kQuarterP>(tmem_base + kColDV, tp, sdo + d2 * SM::kTile, 1, true);
@@ -416,7 +421,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(half == 0 ? &bars->p_half : &bars->p_ready);
+        if (lane == 0) mbar_arrive(half == 0 ? &bars->p_half[t & 1] : &bars->p_ready[t & 1]);
       }
       ok = mbar_wait(&bars->dp_full, par, abort_word, p.status);
       if (!ok) break;
