@@ -152,13 +152,17 @@ constexpr int RMS_BWD_MAX_STAGES = 8;
 // the register-staged version at half the HBM rate (and at d > 4096, where only one block of it
 // fitted, at a fifth).  The barrier of row i+1 also tells that every thread is done with row i,
 // whose stage is refilled right after it.
+// A copy that does not land within the wait's limit is reported through the status word, and the
+// block's rows from there on and the weight gradient become NaN (the entry point without a status
+// word has only that).  Every thread still walks through all rows: none is missing at a barrier.
 // 8192x4096 with dres: 84.6 -> 48.2 us, 8192x5120: 245 -> 66 us, 8192x2048: 49.9 -> 34.8 us.
 template <int NT, int NCH, bool RES>
 __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                       float* __restrict__ dw_partial, int rows, int d, int stages) {
+                       float* __restrict__ dw_partial, int rows, int d, int stages,
+                       int* __restrict__ status) {
   constexpr int NW = NT / 32;
   constexpr int NIN = RES ? 3 : 2;
   extern __shared__ __align__(128) uint8_t ring[];   // [stages][NIN][d] bf16
@@ -183,8 +187,9 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
     mbar_fence_init();
   }
   dep_wait();
+  int filled = stages < n ? stages : n;   // rows whose copies have been issued (thread 0)
   if (threadIdx.x == 0) {
-    for (int it = 0; it < stages && it < n; ++it) fill(it);
+    for (int it = 0; it < filled; ++it) fill(it);
   }
   float acc[NCH][8];
   uint4 wv[NCH];
@@ -197,17 +202,14 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
   }
   __syncthreads();
   float rs_next = n > 0 ? rstd[blockIdx.x] : 0.f;
+  int good = 0;   // rows that have landed; after a failure the thread waits for no further one
   for (int it = 0; it < n; ++it) {
     const int row = (int)blockIdx.x + it * (int)gridDim.x;
     const int st = it % stages;
     const float rs = rs_next;
     if (it + 1 < n) rs_next = rstd[row + gridDim.x];
-    if (!mbar_wait(&full[st], (uint32_t)(it / stages) & 1, &abort_word, nullptr)) {
-      // no status word here: a copy that never landed shows as NaN in the weight gradient
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) acc[ch][0] = __int_as_float(0x7fffffff);
-      break;
-    }
+    if (good == it && mbar_wait(&full[st], (uint32_t)(it / stages) & 1, &abort_word, status))
+      ++good;
     const __nv_bfloat16* sx = reinterpret_cast<const __nv_bfloat16*>(
         ring + (size_t)st * NIN * row_bytes);
     float xh[NCH][8], g[NCH][8];
@@ -229,10 +231,17 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
         }
       }
     }
+    if (good <= it) {
+      dot = __int_as_float(0x7fffffff);
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[ch][i] = dot;
+    }
     dot = warp_sum(dot);
     if (lane == 0) red[it & 1][warp] = dot;
     __syncthreads();
-    if (threadIdx.x == 0 && it > 0 && it - 1 + stages < n) fill(it - 1 + stages);
+    if (threadIdx.x == 0 && it > 0 && filled < n && good > it) fill(filled++);
     dot = 0.f;
 #pragma unroll
     for (int k = 0; k < NW; ++k) dot += red[it & 1][k];
@@ -254,6 +263,13 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
         store8(dxr + c, o);
       }
     }
+  }
+  if (threadIdx.x == 0 && good < n) {   // copies in flight still write to this block's memory
+    const long long t0 = clock64();
+    for (int k = good; k < filled; ++k)
+      while (!mbar_try_wait(&full[k % stages], (uint32_t)(k / stages) & 1) &&
+             clock64() - t0 < MB200_WAIT_CYCLES) {
+      }
   }
   float* out = dw_partial + (size_t)blockIdx.x * d;
 #pragma unroll
@@ -297,7 +313,7 @@ template <int NT, int NCH, bool RES>
 static int launch_rmsnorm_bwd_t(int nb, const __nv_bfloat16* dy, const __nv_bfloat16* x,
                                 const __nv_bfloat16* w, const float* rstd,
                                 const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw_partial,
-                                int rows, int d, cudaStream_t st) {
+                                int rows, int d, int* status, cudaStream_t st) {
   // four blocks of 48 KB, two of 96 or one of 192 per SM
   constexpr int kRing = NT * NCH * 192;
   static bool configured = false;
@@ -311,7 +327,7 @@ static int launch_rmsnorm_bwd_t(int nb, const __nv_bfloat16* dy, const __nv_bflo
   int stages = kRing / stage;
   if (stages > RMS_BWD_MAX_STAGES) stages = RMS_BWD_MAX_STAGES;
   return (int)launch_dep(rmsnorm_bwd_kernel<NT, NCH, RES>, nb, NT, stages * stage, st, dy, x, w,
-                         rstd, dres, dx, dw_partial, rows, d, stages);
+                         rstd, dres, dx, dw_partial, rows, d, stages, status);
 }
 
 // Launches the backward pair: nb row-striding blocks (fewer where one block fills an SM), then
@@ -319,16 +335,16 @@ static int launch_rmsnorm_bwd_t(int nb, const __nv_bfloat16* dy, const __nv_bflo
 static int launch_rmsnorm_bwd(int nb, const __nv_bfloat16* dy, const __nv_bfloat16* x,
                               const __nv_bfloat16* w, const float* rstd,
                               const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw_partial,
-                              __nv_bfloat16* dw, int dw_accumulate, int rows, int d,
+                              __nv_bfloat16* dw, int dw_accumulate, int rows, int d, int* status,
                               cudaStream_t st) {
   int rc;
   const int resident = d > 4096 ? 148 : d > 2048 ? 296 : 592;
   if (nb > resident) nb = resident;
 #define MB200_RMS_BWD(NT, NCH)                                                                  \
   (dres ? launch_rmsnorm_bwd_t<NT, NCH, true>(nb, dy, x, w, rstd, dres, dx, dw_partial, rows, d, \
-                                              st)                                               \
+                                              status, st)                                       \
         : launch_rmsnorm_bwd_t<NT, NCH, false>(nb, dy, x, w, rstd, dres, dx, dw_partial, rows, d, \
-                                               st))
+                                               status, st))
   if (d <= 2048)
     rc = MB200_RMS_BWD(256, 1);
   else if (d <= 4096)
@@ -741,12 +757,13 @@ extern "C" int mb200_rmsnorm_bwd_blocks(int rows) {
 
 extern "C" int mb200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
                                  const void* dres, void* dx, float* dw_partial, void* dw,
-                                 int dw_accumulate, int rows, int d, void* stream) {
+                                 int dw_accumulate, int rows, int d, int* status,
+                                 void* stream) {
   if (rows <= 0) return 0;
   if (d % 8 || d > RMS_BWD_MAX_D) return 1001;
   const int nb = mb200_rmsnorm_bwd_blocks(rows);
   return launch_rmsnorm_bwd(nb, CBF(dy), CBF(x), CBF(w), rstd, CBF(dres), BF(dx), dw_partial,
-                            BF(dw), dw_accumulate, rows, d, ST(stream));
+                            BF(dw), dw_accumulate, rows, d, status, ST(stream));
 }
 
 extern "C" int mb200_rope_inplace(void* qkv, const float* cos_t, const float* sin_t, int rows,
@@ -899,5 +916,5 @@ extern "C" int mb200_rmsnorm_bwd_noalloc(const void* dy, const void* x, const vo
   const int cap = MB200_NOALLOC_SCRATCH_FLOATS / d;
   if (nb > cap) nb = cap;
   return launch_rmsnorm_bwd(nb, CBF(dy), CBF(x), CBF(w), rstd, CBF(dres), BF(dx), scratch, BF(dw),
-                            dw_accumulate, rows, d, ST(stream));
+                            dw_accumulate, rows, d, /*status=*/nullptr, ST(stream));
 }

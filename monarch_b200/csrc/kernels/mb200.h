@@ -39,7 +39,7 @@ int mb200_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int ro
 int mb200_rmsnorm_bwd_blocks(int rows);
 int mb200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
                       const void* dres, void* dx, float* dw_partial, void* dw, int dw_accumulate,
-                      int rows, int d, void* stream);
+                      int rows, int d, int* status, void* stream);
 
 // In-place rotary embedding (rotate-half convention) on the first n_rot_heads heads of
 // each row of `qkv` ([rows, row_stride] bf16, head h at columns [h*hd, (h+1)*hd)).

@@ -111,7 +111,7 @@ def rmsnorm_bwd(dy, x, w, rstd, dw_out, accumulate=False, dres=None):
     part = _rms_scratch(x.device, nb, d)
     K.check(K.lib().mb200_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(),
                                       _p(dres), dx.data_ptr(), part.data_ptr(), dw_out.data_ptr(),
-                                      int(accumulate), rows, d, K.stream_ptr()),
+                                      int(accumulate), rows, d, K.status_ptr(x), K.stream_ptr()),
             "rmsnorm_bwd", 2)
     return dx
 

@@ -62,7 +62,7 @@ def _declare(l: ctypes.CDLL) -> None:
                                   _vp]
     l.mb200_rmsnorm_fwd.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _f, _vp]
     l.mb200_rmsnorm_bwd_blocks.argtypes = [_i]
-    l.mb200_rmsnorm_bwd.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]
+    l.mb200_rmsnorm_bwd.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp]
     l.mb200_rope_inplace.argtypes = [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]
     l.mb200_swiglu_fwd.argtypes = [_vp, _vp, _i, _i, _vp]
     l.mb200_swiglu_bwd.argtypes = [_vp, _vp, _vp, _i, _i, _vp]

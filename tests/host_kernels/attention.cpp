@@ -1,4 +1,4 @@
-// Runs an attention kernel's source under many schedules (tests/test_attention_handshake.py).
+// Runs an attention kernel's source under many schedules (tests/test_kernel_waits.py).
 // Arguments: head size, warps of a block, seeds per actor that is held back.
 #include KERNEL_SOURCE
 

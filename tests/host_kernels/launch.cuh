@@ -5,7 +5,7 @@
 
 namespace hostsim {
 inline unsigned g_seed = 0;
-inline int g_starved = -1;
+inline int g_starved = -1, g_drop = -1;
 inline std::string g_error;
 }  // namespace hostsim
 
@@ -14,9 +14,10 @@ static inline void dep_wait() {}
 static inline void dep_launch() {}
 
 template <typename... P, typename... A>
-static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t, cudaStream_t,
-                              A&&... args) {
-  if (block.x == 256) return cudaSuccess;   // element-wise: no barriers to check
+static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem_bytes,
+                              cudaStream_t, A&&... args) {
+  if (smem_bytes == 0) return cudaSuccess;   // no pipeline to check
+  gridDim.x = grid.x;
   for (unsigned z = 0; z < grid.z; ++z)
     for (unsigned y = 0; y < grid.y; ++y)
       for (unsigned x = 0; x < grid.x; ++x) {
@@ -24,7 +25,7 @@ static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_
         blockIdx.y = y;
         blockIdx.z = z;
         const std::string e = hostsim::run_block(block.x / 32, hostsim::g_seed, hostsim::g_starved,
-                                                 [&] { kernel(args...); });
+                                                 hostsim::g_drop, [&] { kernel(args...); });
         if (!e.empty()) {
           hostsim::g_error = "block " + std::to_string(x) + "," + std::to_string(y) + ": " + e;
           return cudaErrorUnknown;
