@@ -82,18 +82,6 @@ def rmsnorm_fwd(x, w, eps=1e-5):
     return y, rstd
 
 
-_scratch: dict = {}
-
-
-def _rms_scratch(device, nblocks, d):
-    key = (device, "rms")
-    t = _scratch.get(key)
-    if t is None or t.numel() < nblocks * d:
-        t = torch.empty(nblocks * d, dtype=torch.float32, device=device)
-        _scratch[key] = t
-    return t
-
-
 def rmsnorm_bwd(dy, x, w, rstd, dw_out, accumulate=False, dres=None):
     """Returns dx (+ ``dres``); writes (or adds) the weight gradient into ``dw_out``."""
     rows, d = x.shape
@@ -108,7 +96,8 @@ def rmsnorm_bwd(dy, x, w, rstd, dw_out, accumulate=False, dres=None):
     dy = dy.contiguous()
     dx = torch.empty_like(x)
     nb = K.lib().mb200_rmsnorm_bwd_blocks(rows)
-    part = _rms_scratch(x.device, nb, d)
+    # of this call alone: another stream's call may run between the two kernels that use it
+    part = torch.empty(nb * d, dtype=torch.float32, device=x.device)
     K.check(K.lib().mb200_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(),
                                       _p(dres), dx.data_ptr(), part.data_ptr(), dw_out.data_ptr(),
                                       int(accumulate), rows, d, K.status_ptr(x), K.stream_ptr()),

@@ -358,3 +358,29 @@ def test_gemm_swiglu_equals_the_separate_kernels(gemm_impl, T, F, K_):
     wd = (0.1 * torch.randn(K_, F, device="cuda")).to(bf16)
     ref = ops.swiglu_bwd(gu, ops.gemm(dy, wd, b_mn=True))
     assert _rel(ops.gemm_swiglu_bwd(dy, wd, gu), ref) < 1e-3
+
+
+def test_rmsnorm_bwd_on_two_streams_shares_no_scratch(monkeypatch):
+    """The partial weight-gradient sums of a call are read by its second kernel, while a call on
+    another stream may already write its own."""
+    lib, used = K.lib(), []
+
+    class Recorder:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def mb200_rmsnorm_bwd(self, *args):
+            used.append(args[6])
+            return lib.mb200_rmsnorm_bwd(*args)
+
+    monkeypatch.setattr(K, "lib", lambda: Recorder())
+    x = torch.randn(64, 512, device="cuda", dtype=bf16)
+    w = torch.ones(512, device="cuda", dtype=bf16)
+    _, rstd = ops.rmsnorm_fwd(x, w, 1e-5)
+    dw = torch.empty(2, 512, device="cuda", dtype=bf16)
+    torch.cuda.synchronize()
+    for i, st in enumerate((torch.cuda.Stream(), torch.cuda.Stream())):
+        with torch.cuda.stream(st):
+            ops.rmsnorm_bwd(x, x, w, rstd, dw[i])
+    torch.cuda.synchronize()
+    assert len(set(used)) == 2 and torch.equal(dw[0], dw[1])
