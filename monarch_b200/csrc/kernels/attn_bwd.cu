@@ -724,17 +724,11 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
 template <int HD>
 static int launch_attn_bwd(const void* q, const void* k, const void* v, const void* dout,
                            int ld_qkv, int ld_do, const AttBwdParams& p, cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_dkv_kernel<HD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         AbSmem<HD>::kTotal);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_bwd_dq_kernel<HD>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, AbSmem<HD>::kTotal);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static PerDevice<int> dkv_smem_ok, dq_smem_ok;
+  if (const cudaError_t e = allow_smem(attn_bwd_dkv_kernel<HD>, AbSmem<HD>::kTotal, dkv_smem_ok))
+    return (int)e;
+  if (const cudaError_t e = allow_smem(attn_bwd_dq_kernel<HD>, AbSmem<HD>::kTotal, dq_smem_ok))
+    return (int)e;
   const uint64_t T = (uint64_t)p.B * p.S;
   CUtensorMap tq, tk, tv, tdo;   // boxes of 64 columns x 128 rows
   int r = make_tmap_bf16_2d(&tq, q, (uint64_t)p.Hq * HD, T, ld_qkv, 64, AB_T);

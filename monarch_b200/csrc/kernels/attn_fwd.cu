@@ -404,13 +404,8 @@ template <int HD>
 static int launch_attn_fwd(const void* q, const void* k, const void* v, const AttFwdParams& p,
                            int ld_qkv, cudaStream_t st) {
   using SM = AttFwdSmem<HD>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<HD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kTotal);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static PerDevice<int> smem_ok;
+  if (const cudaError_t e = allow_smem(attn_fwd_kernel<HD>, SM::kTotal, smem_ok)) return (int)e;
   const uint64_t T = (uint64_t)p.B * p.S;
   CUtensorMap tq, tk, tv;
   int r = make_tmap_bf16_2d(&tq, q, (uint64_t)p.Hq * HD, T, ld_qkv, 64, ATT_BM);

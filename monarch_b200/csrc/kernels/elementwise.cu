@@ -316,13 +316,9 @@ static int launch_rmsnorm_bwd_t(int nb, const __nv_bfloat16* dy, const __nv_bflo
                                 int rows, int d, int* status, cudaStream_t st) {
   // four blocks of 48 KB, two of 96 or one of 192 per SM
   constexpr int kRing = NT * NCH * 192;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_kernel<NT, NCH, RES>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kRing);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static PerDevice<int> smem_ok;
+  if (const cudaError_t e = allow_smem(rmsnorm_bwd_kernel<NT, NCH, RES>, kRing, smem_ok))
+    return (int)e;
   const int stage = (RES ? 3 : 2) * d * 2;
   int stages = kRing / stage;
   if (stages > RMS_BWD_MAX_STAGES) stages = RMS_BWD_MAX_STAGES;

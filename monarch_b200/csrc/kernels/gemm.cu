@@ -46,13 +46,16 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64
 }
 
 int sm_count() {
-  static int n = 0;
-  if (!n) {
+  static PerDevice<int> known;
+  int* n = known.here();
+  int now = n ? *n : 0;
+  if (!now) {
     int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&now, cudaDevAttrMultiProcessorCount, dev);
+    if (n) *n = now;
   }
-  return n;
+  return now;
 }
 
 template <bool A_MN, bool B_MN, int BN, int EPI>
@@ -66,14 +69,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 template <bool A_MN, bool B_MN, int BN, int EPI = kEpiStore>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
                   cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         GemmTile<BN>::kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static PerDevice<int> smem_ok;
+  if (const cudaError_t e =
+          allow_smem(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>, GemmTile<BN>::kSmemBytes, smem_ok))
+    return (int)e;
   return (int)launch_dep(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>, grid, GEMM_THREADS,
                          GemmTile<BN>::kSmemBytes, st, ta, tb, p);
 }
@@ -286,11 +285,12 @@ __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 // Number of clusters of SPLIT CTAs that can be resident at once; 0 when there is no answer.
 template <bool A_MN, bool B_MN, int BN, int SPLIT>
 static int split_capacity() {
-  static int cap = -1;
-  if (cap >= 0) return cap;
-  if (cudaFuncSetAttribute(gemm_split_kernel<A_MN, B_MN, BN, SPLIT>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           GemmTile<BN>::kSmemBytes) != cudaSuccess) {
+  static PerDevice<int> known;   // capacity + 1
+  int* cap = known.here();
+  if (cap && *cap) return *cap - 1;
+  static PerDevice<int> smem_ok;
+  if (allow_smem(gemm_split_kernel<A_MN, B_MN, BN, SPLIT>, GemmTile<BN>::kSmemBytes, smem_ok) !=
+      cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -311,8 +311,8 @@ static int split_capacity() {
     cudaGetLastError();
     n = 0;
   }
-  cap = n;
-  return cap;
+  if (cap) *cap = n + 1;
+  return n;
 }
 
 template <bool A_MN, bool B_MN, int BN, int SPLIT>
@@ -351,11 +351,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm2_threads(EPI), 
 // odd number of usable SMs).  Queried once per operand-layout variant.
 template <bool A_MN, bool B_MN, int EPI>
 static int pair_capacity() {
-  static int cap = 0;
-  if (cap) return cap;
-  if (cudaFuncSetAttribute(gemm2_bf16_kernel<A_MN, B_MN, EPI>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           G2_SMEM_BYTES) != cudaSuccess)
+  static PerDevice<int> known, smem_ok;
+  int* cap = known.here();
+  if (cap && *cap) return *cap;
+  if (allow_smem(gemm2_bf16_kernel<A_MN, B_MN, EPI>, G2_SMEM_BYTES, smem_ok) != cudaSuccess)
     return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (sm_count() / 2));
@@ -375,8 +374,8 @@ static int pair_capacity() {
     n = sm_count() / 2;
   }
   if (n > sm_count() / 2) n = sm_count() / 2;
-  cap = n;
-  return cap;
+  if (cap) *cap = n;
+  return n;
 }
 
 template <bool A_MN, bool B_MN, int EPI = kEpiStore>

@@ -20,6 +20,8 @@
 
 #include <utility>
 
+#include "per_device.cuh"
+
 namespace mb200 {
 
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -334,17 +334,10 @@ extern "C" int mb200_moe_gather_gemm(const void* const* counts_ptrs, const void*
     int pairs = sms / 2 - n_comm / 2;
     if (tiles < pairs) pairs = tiles;
     const int grid = n_comm + 2 * pairs;
-    static bool configured2[2] = {false, false};
-    if (!configured2[b_mn ? 1 : 0]) {
-      cudaError_t e = b_mn ? cudaFuncSetAttribute(moe_gather_gemm_pair_kernel<true>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  G2_SMEM_BYTES)
-                           : cudaFuncSetAttribute(moe_gather_gemm_pair_kernel<false>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  G2_SMEM_BYTES);
-      if (e != cudaSuccess) return (int)e;
-      configured2[b_mn ? 1 : 0] = true;
-    }
+    static PerDevice<int> smem_ok[2];
+    if (const cudaError_t e = allow_smem(b_mn ? moe_gather_gemm_pair_kernel<true> : moe_gather_gemm_pair_kernel<false>,
+                                         G2_SMEM_BYTES, smem_ok[b_mn ? 1 : 0]))
+      return (int)e;
     if (b_mn)
       moe_gather_gemm_pair_kernel<true><<<grid, GEMM_THREADS, G2_SMEM_BYTES, st>>>(ta2, tb2, p, g,
                                                                                   n_comm);
@@ -356,17 +349,10 @@ extern "C" int mb200_moe_gather_gemm(const void* const* counts_ptrs, const void*
   const int tiles = ((cap + GEMM_BM - 1) / GEMM_BM) * ((N + GEMM_BN - 1) / GEMM_BN);
   int gemm_ctas = sms - n_comm;
   if (tiles < gemm_ctas) gemm_ctas = tiles;
-  static bool configured[2] = {false, false};
-  if (!configured[b_mn ? 1 : 0]) {
-    cudaError_t e = b_mn ? cudaFuncSetAttribute(moe_gather_gemm_kernel<true>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                GEMM_SMEM_BYTES)
-                         : cudaFuncSetAttribute(moe_gather_gemm_kernel<false>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                GEMM_SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    configured[b_mn ? 1 : 0] = true;
-  }
+  static PerDevice<int> smem_ok[2];
+  if (const cudaError_t e = allow_smem(b_mn ? moe_gather_gemm_kernel<true> : moe_gather_gemm_kernel<false>,
+                                       GEMM_SMEM_BYTES, smem_ok[b_mn ? 1 : 0]))
+    return (int)e;
   const int grid = n_comm + gemm_ctas;
   if (b_mn)
     moe_gather_gemm_kernel<true><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb, p, g, n_comm);

@@ -25,6 +25,7 @@ int main(int, char** argv) {
     for (int seed = 0; seed < n_seeds; ++seed) {
       hostsim::g_seed = (unsigned)seed;
       hostsim::g_starved = starved;
+      hostsim::g_device = seed & 1;
 #ifdef BACKWARD
       const int rc = mb200_attn_bwd(qkv.data(), qkv.data(), qkv.data(), ob, ob, up16(lse.data()),
                                     up16(delta.data()), dq, dq + Hq * hd, dq + (Hq + Hkv) * hd, B, S,

@@ -2,6 +2,7 @@
 // under the schedule that is set.
 #pragma once
 #include "ptx.cuh"
+#include PER_DEVICE_HEADER
 
 namespace hostsim {
 inline unsigned g_seed = 0;
@@ -17,6 +18,11 @@ template <typename... P, typename... A>
 static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem_bytes,
                               cudaStream_t, A&&... args) {
   if (smem_bytes == 0) return cudaSuccess;   // no pipeline to check
+  if (smem_bytes > 48 * 1024 &&
+      (size_t)hostsim::g_allowed[{(const void*)kernel, hostsim::g_device}] < smem_bytes) {
+    hostsim::g_error = "the kernel may not use that much shared memory on this device";
+    return cudaErrorInvalidValue;
+  }
   gridDim.x = grid.x;
   for (unsigned z = 0; z < grid.z; ++z)
     for (unsigned y = 0; y < grid.y; ++y)

@@ -199,8 +199,20 @@ static inline long long clock64() {
   return t += 100;
 }
 #define MB200_WAIT_CYCLES 100000
+// Two devices: what a kernel may use on one says nothing about the other.
+namespace hostsim {
+static int g_device = 0;
+static std::map<std::pair<const void*, int>, int> g_allowed;
+}  // namespace hostsim
+extern "C" cudaError_t cudaGetDevice(int* dev) {
+  *dev = hostsim::g_device;
+  return cudaSuccess;
+}
 template <typename F>
-static cudaError_t cudaFuncSetAttribute(F*, cudaFuncAttribute, int) { return cudaSuccess; }
+static cudaError_t cudaFuncSetAttribute(F* kernel, cudaFuncAttribute, int bytes) {
+  hostsim::g_allowed[{(const void*)kernel, hostsim::g_device}] = bytes;
+  return cudaSuccess;
+}
 
 namespace mb200 {
 inline uint8_t smem[232448] __attribute__((aligned(1024)));       // dynamic shared memory, by the

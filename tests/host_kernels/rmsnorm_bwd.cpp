@@ -18,6 +18,7 @@ int main(int, char** argv) {
       for (int res = 0; res < 2; ++res) {
         hostsim::g_seed = (unsigned)seed;
         hostsim::g_starved = starved;
+        hostsim::g_device = seed & 1;
         hostsim::g_drop = drop;
         int status = 0;
         const auto untouched = __float2bfloat16(7.f);

@@ -1,7 +1,8 @@
 """The waits inside pipelined kernels, on the CPU: the kernels' own sources run under stand-ins for
 the hardware's barriers (tests/host_kernels), with schedules that hold back each warp, the tensor
 pipe or the TMA unit for as long as any other can go on.  A wait that is right only because one
-side is fast enough in practice misses its phase in one of them."""
+side is fast enough in practice misses its phase in one of them.  The launches alternate between
+two devices, whose kernels need their shared memory allowed one by one."""
 import re
 import shutil
 import subprocess
@@ -26,7 +27,7 @@ def _build(tmp, source, text, driver):
         shutil.copy(HOST / f, tmp / f)
     shutil.copy(KERNELS / "mb200.h", tmp / "mb200.h")
     cmd = ["g++", "-std=c++17", "-O1", "-w", f"-I{CUDA}", "-x", "c++",
-           f'-DKERNEL_SOURCE="{source}"', *(["-DBACKWARD"] if "bwd" in source else []),
+           f'-DPER_DEVICE_HEADER="{KERNELS / "per_device.cuh"}"', f'-DKERNEL_SOURCE="{source}"', *(["-DBACKWARD"] if "bwd" in source else []),
            driver, "-o", "run"]
     p = subprocess.run(cmd, cwd=tmp, capture_output=True, text=True)
     assert p.returncode == 0, p.stderr[-3000:]
