@@ -77,7 +77,9 @@ def run_arm(mesh, impl: str, args, e2e: bool):
     from monarch_b200.parallel.trainer_actor import TrainerActor
     spec = {"impl": impl, "model": args.model, "seq_len": args.seq, "micro_batch": args.micro_batch,
             "parallelism": args.parallelism, "comm": args.comm,
-            "recompute_layers": args.recompute_layers, "microbatches": args.microbatches,
+            "recompute_layers": args.recompute_layers,
+            "keep_residual": True,   # 2 of 183 GB at the default size
+            "microbatches": args.microbatches,
             "schedule": args.schedule, "cuda": not args.cpu}
     trainers = mesh.spawn(f"trainer_{impl}", TrainerActor, spec)
     info = [v for _, v in trainers.info.call().get(timeout=1800).items()]

@@ -348,10 +348,12 @@ class LlamaEngine:
     """
 
     def __init__(self, cfg: LlamaConfig, store, seq_len: int, checkpoint: bool = True,
-                 recompute_layers: Optional[int] = None):
+                 recompute_layers: Optional[int] = None, keep_residual: bool = False):
         """``checkpoint``: keep only each layer's input (and, with the attention kernels, its
-        attention output and the residual stream behind it) in the forward and recompute the
-        rest in the backward.  ``recompute_layers`` (with ``checkpoint``):
+        attention output) in the forward and recompute the rest in the backward.
+        ``keep_residual`` (with both): also keep the residual stream behind the attention, 2
+        more bytes per token and model-dim element of each recomputed layer, so that the
+        output projection is not run again.  ``recompute_layers`` (with ``checkpoint``):
         how many of the layers, counted from the first, are treated that way; the remaining
         last layers keep all their activations (about 17 bytes per token per model-dim
         element each), trading spare HBM for one skipped forward per kept layer.  Default:
@@ -366,18 +368,19 @@ class LlamaEngine:
         dev = store.device
         self.cos, self.sin = ops.reference.rope_tables(seq_len, cfg.hd, cfg.theta, device=dev)
         self.n_units = cfg.n_layers + 2
-        # with checkpointing, keep each layer's attention output, log-sum-exp and residual
-        # stream so the recompute pass skips the attention kernel and projection (only with the hand-written kernels,
+        # with checkpointing, keep each layer's attention output and log-sum-exp so the
+        # recompute pass skips the attention kernel (only with the hand-written kernels,
         # whose backward needs nothing else from the forward)
         self.keep_attention = checkpoint and ops.have_attention_kernel() and \
             torch.device(dev).type == "cuda"
+        self.keep_residual = keep_residual and self.keep_attention
 
     # ------------------------------------------------------------------ layer forward
     def _attn_fwd(self, w: dict, x: torch.Tensor, B: int, S: int, keep: bool, attn_saved=None):
-        """x -> x + attention(norm(x)).  ``attn_saved`` = (o, lse, x2) kept from the first
-        forward: the recompute pass then rebuilds q/k/v but runs neither the attention kernel
-        nor the output projection again (selective checkpointing: 4 bytes per activation
-        element per layer; the projection alone is 2 % of a checkpointed layer's FLOPs)."""
+        """x -> x + attention(norm(x)).  ``attn_saved`` = (o, lse, x2 or None) kept from the
+        first forward: the recompute pass then rebuilds q/k/v but does not run the attention
+        kernel again (selective checkpointing: 2 bytes per activation element per layer), and
+        with x2 (2 bytes more) not the output projection either, 2 % of a layer's FLOPs."""
         cfg = self.cfg
         h1, rstd1 = ops.rmsnorm_fwd(x, w["attn_norm"], cfg.eps)
         qkv = _unit_gemm(w, h1, "wqkv")
@@ -385,7 +388,8 @@ class LlamaEngine:
         if attn_saved is not None:
             attn, actx = ops.attention_ctx_from_saved(qkv, attn_saved[:2], B, S, cfg.n_heads,
                                                       cfg.n_kv_heads, cfg.hd)
-            return attn_saved[2], (x, rstd1, h1, actx, attn)
+            if attn_saved[2] is not None:
+                return attn_saved[2], (x, rstd1, h1, actx, attn)
         else:
             attn, actx = ops.attention_fwd(qkv, B, S, cfg.n_heads, cfg.n_kv_heads, cfg.hd,
                                            need_bwd=keep or self.keep_attention)
@@ -412,7 +416,7 @@ class LlamaEngine:
             return y, (sa, sm)
         actx = sa[3]
         if self.keep_attention and actx.lse is not None:
-            return y, (actx.o, actx.lse, x2)
+            return y, (actx.o, actx.lse, x2 if self.keep_residual else None)
         return y, None
 
     def _mlp_bwd(self, w: dict, g: dict, sm, dy: torch.Tensor):

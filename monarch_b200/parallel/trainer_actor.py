@@ -32,7 +32,8 @@ class TrainerActor(Actor):
     def __init__(self, spec: Dict[str, Any]):
         """``spec``: ``impl`` ("ours" | "aten"), ``model``, ``seq_len``, ``micro_batch``,
         ``parallelism`` ("auto", "single", "fsdp", "ddp", "ep", "ppPxtpT"), ``comm``,
-        ``recompute_layers``, ``microbatches``, ``schedule``, ``n_batches``, ``cuda``."""
+        ``recompute_layers``, ``keep_residual``, ``microbatches``, ``schedule``, ``n_batches``,
+        ``cuda``."""
         self.spec = dict(spec)
         self.rank = current_rank().rank
         self.world = 1
@@ -84,6 +85,7 @@ class TrainerActor(Actor):
             self.trainer = Trainer(model, seq_len=seq, micro_batch=mb, parallelism=par,
                                    device=self.device, comm=comm,
                                    recompute_layers=s.get("recompute_layers"),
+                                   keep_residual=bool(s.get("keep_residual", False)),
                                    lr=float(s.get("lr", 3e-4)))
         self._pipeline = bool(m_pp)
         cfg = self.trainer.cfg
