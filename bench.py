@@ -185,8 +185,9 @@ def main():
         "loss": res["loss"], "max_mem_gb": res["max_mem_gb"],
         # model FLOPs (3x forward; recomputation not counted) and what the hardware executed
         "model_tflops_per_gpu": cfg.flops_per_token(S) * per_gpu / 1e12,
-        "hardware_tflops_per_gpu": cfg.flops_per_token(S, recompute=True) * per_gpu / 1e12
-        if args.recompute_layers is None else None,
+        # (of LlamaEngine; the pipeline's stages recompute differently)
+        "hardware_tflops_per_gpu": cfg.flops_per_token(S, recompute=True, keep_residual=True) *
+        per_gpu / 1e12 if args.recompute_layers is None and not m_pp else None,
         "baseline": None if base is None else {
             "impl": "aten: stock torch modules (cuBLAS, SDPA), autograd checkpointing, fused "
                     "torch AdamW on fp32 masters" + ("; fully_shard over NCCL" if world > 1 else ""),

@@ -3,8 +3,8 @@ model (same weights, fp32 CPU reference ops)."""
 import pytest
 import torch
 
-from monarch_b200.models import (PRESETS, LlamaEngine, LocalParamStore, ParamLayout, TorchLlama,
-                                 load_hf_state_dict, to_hf_state_dict)
+from monarch_b200.models import (PRESETS, LlamaConfig, LlamaEngine, LocalParamStore, ParamLayout,
+                                 TorchLlama, load_hf_state_dict, to_hf_state_dict)
 
 
 def _fp32_store(cfg, layout):
@@ -69,3 +69,38 @@ def test_adamw_step_matches_torch():
         opt.step()
         st.optimizer_step(1e-3)
     assert torch.allclose(st.master, p.detach(), atol=1e-6)
+
+
+@pytest.mark.parametrize("checkpoint,keep_residual", [(True, False), (True, True), (False, False)])
+def test_flops_per_token_counts_the_products_that_run(monkeypatch, checkpoint, keep_residual):
+    """The FLOPs of all products of a pass, counted at the call; attention by its own formula."""
+    from monarch_b200 import ops
+    cfg = LlamaConfig(vocab=96, d=64, n_layers=3, n_heads=4, n_kv_heads=2, ffn=160)
+    st = LocalParamStore(ParamLayout(cfg), "cpu", seed=0)
+    eng = LlamaEngine(cfg, st, seq_len=16, checkpoint=checkpoint)
+    # as with the attention kernels, whose output and log-sum-exp are kept
+    eng.keep_attention, eng.keep_residual = checkpoint, keep_residual
+    attend = ops.attention_fwd
+
+    def attention_fwd(*a, **kw):
+        o, ctx = attend(*a, **kw)
+        ctx.lse = torch.zeros(1)
+        return o, ctx
+
+    monkeypatch.setattr(ops, "attention_fwd", attention_fwd)
+    monkeypatch.setattr(ops, "attention_bwd", lambda ctx, do: torch.zeros_like(ctx.qkv))
+    total = [0]
+    gemm = ops.gemm
+
+    def counted(a, b, a_mn=False, b_mn=False, **kw):
+        out = gemm(a, b, a_mn=a_mn, b_mn=b_mn, **kw)
+        total[0] += 2 * out.shape[0] * out.shape[1] * (a.shape[0] if a_mn else a.shape[1])
+        return out
+
+    monkeypatch.setattr(ops, "gemm", counted)
+    monkeypatch.setattr(ops.functional, "gemm", counted)
+    tok = torch.randint(0, cfg.vocab, (2, 16))
+    eng.forward_backward(tok, tok)
+    attn = cfg.n_layers * 2 * 16 * cfg.d * (3.5 if checkpoint else 3)
+    want = cfg.flops_per_token(16, recompute=checkpoint, keep_residual=keep_residual) - attn
+    assert total[0] == want * tok.numel()
