@@ -766,7 +766,7 @@ extern "C" int mb200_rope_inplace(void* qkv, const float* cos_t, const float* si
                                   int seq_len, int n_rot_heads, int hd, int row_stride,
                                   int inverse, void* stream) {
   if (rows <= 0) return 0;
-  if (hd % 16 || row_stride % 8) return 1001;
+  if (hd % 16 || row_stride % 8 || hd <= 0 || n_rot_heads <= 0) return 1001;
   if (hd <= 512 && (hd & (hd - 1)) == 0 && aligned16(cos_t) && aligned16(sin_t)) {
     return (int)launch_dep(rope_row_kernel, blocks_for(rows, 32 / (hd / 16)), 256, 0, ST(stream),
                            BF(qkv), cos_t, sin_t, rows, seq_len, n_rot_heads, __builtin_ctz(hd),
@@ -779,8 +779,7 @@ extern "C" int mb200_rope_inplace(void* qkv, const float* cos_t, const float* si
 
 extern "C" int mb200_swiglu_fwd(const void* gu, void* h, int rows, int F, void* stream) {
   if (rows <= 0) return 0;
-  if (F % 8) return 1001;
-  if (F <= 0) return 0;
+  if (F % 8 || F <= 0) return 1001;
   const int nt = row_threads(F / 8);
   return (int)launch_dep(swiglu_fwd_kernel, dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream),
                          CBF(gu), BF(h), F);
@@ -788,8 +787,7 @@ extern "C" int mb200_swiglu_fwd(const void* gu, void* h, int rows, int F, void* 
 extern "C" int mb200_swiglu_bwd(const void* gu, const void* dh, void* dgu, int rows, int F,
                                 void* stream) {
   if (rows <= 0) return 0;
-  if (F % 8) return 1001;
-  if (F <= 0) return 0;
+  if (F % 8 || F <= 0) return 1001;
   const int nt = row_threads(F / 8);
   return (int)launch_dep(swiglu_bwd_kernel, dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream),
                          CBF(gu), CBF(dh), BF(dgu), F);
@@ -832,8 +830,7 @@ extern "C" int mb200_embedding_fwd(const void* table, const int64_t* ids, void* 
 extern "C" int mb200_embedding_bwd(const void* dout, const int64_t* ids, void* dtable, int rows,
                                    int d, void* stream) {
   if (rows <= 0) return 0;
-  if (d % 2) return 1001;
-  if (d <= 0) return 0;
+  if (d % 2 || d <= 0) return 1001;
   if (d % 8 == 0 && aligned16(dout) && aligned16(dtable)) {
     const int nt = row_threads(d / 8);
     return (int)launch_dep(embedding_bwd_vec_kernel, dim3(rows, blocks_for(d / 8, nt)), nt, 0,
