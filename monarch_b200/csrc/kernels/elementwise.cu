@@ -187,9 +187,8 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
     mbar_fence_init();
   }
   dep_wait();
-  int filled = stages < n ? stages : n;   // rows whose copies have been issued (thread 0)
   if (threadIdx.x == 0) {
-    for (int it = 0; it < filled; ++it) fill(it);
+    for (int it = 0; it < stages && it < n; ++it) fill(it);
   }
   float acc[NCH][8];
   uint4 wv[NCH];
@@ -202,14 +201,15 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
   }
   __syncthreads();
   float rs_next = n > 0 ? rstd[blockIdx.x] : 0.f;
-  int good = 0;   // rows that have landed; after a failure the thread waits for no further one
+  int lost = n;   // the first row that did not land
   for (int it = 0; it < n; ++it) {
     const int row = (int)blockIdx.x + it * (int)gridDim.x;
     const int st = it % stages;
     const float rs = rs_next;
     if (it + 1 < n) rs_next = rstd[row + gridDim.x];
-    if (good == it && mbar_wait(&full[st], (uint32_t)(it / stages) & 1, &abort_word, status))
-      ++good;
+    // (without the status word: polling it in the wait cost up to 8 %)
+    if (lost == n && !mbar_wait(&full[st], (uint32_t)(it / stages) & 1, &abort_word, nullptr))
+      lost = it;
     const __nv_bfloat16* sx = reinterpret_cast<const __nv_bfloat16*>(
         ring + (size_t)st * NIN * row_bytes);
     float xh[NCH][8], g[NCH][8];
@@ -231,17 +231,10 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
         }
       }
     }
-    if (good <= it) {
-      dot = __int_as_float(0x7fffffff);
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[ch][i] = dot;
-    }
-    dot = warp_sum(dot);
+    dot = warp_sum(lost <= it ? __int_as_float(0x7fffffff) : dot);
     if (lane == 0) red[it & 1][warp] = dot;
     __syncthreads();
-    if (threadIdx.x == 0 && it > 0 && filled < n && good > it) fill(filled++);
+    if (threadIdx.x == 0 && it > 0 && it - 1 + stages < n && lost > it) fill(it - 1 + stages);
     dot = 0.f;
 #pragma unroll
     for (int k = 0; k < NW; ++k) dot += red[it & 1][k];
@@ -264,12 +257,19 @@ __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
       }
     }
   }
-  if (threadIdx.x == 0 && good < n) {   // copies in flight still write to this block's memory
-    const long long t0 = clock64();
-    for (int k = good; k < filled; ++k)
-      while (!mbar_try_wait(&full[k % stages], (uint32_t)(k / stages) & 1) &&
-             clock64() - t0 < MB200_WAIT_CYCLES) {
-      }
+  if (lost < n) {
+    if (status) atomicCAS(status, kStatusOk, kStatusMbarTimeout);
+#pragma unroll
+    for (int ch = 0; ch < NCH; ++ch)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[ch][i] = __int_as_float(0x7fffffff);
+    if (threadIdx.x == 0) {   // copies in flight still write to this block's memory
+      const long long t0 = clock64();
+      for (int k = lost; k < n && k < stages + (lost > 0 ? lost - 1 : 0); ++k)
+        while (!mbar_try_wait(&full[k % stages], (uint32_t)(k / stages) & 1) &&
+               clock64() - t0 < MB200_WAIT_CYCLES) {
+        }
+    }
   }
   float* out = dw_partial + (size_t)blockIdx.x * d;
 #pragma unroll

@@ -214,7 +214,15 @@ static cudaError_t cudaFuncSetAttribute(F* kernel, cudaFuncAttribute, int bytes)
   return cudaSuccess;
 }
 
+static inline int atomicCAS(int* p, int want, int now) {
+  const int was = *p;
+  if (was == want) *p = now;
+  return was;
+}
+
 namespace mb200 {
+enum : int { kStatusOk = 0, kStatusMbarTimeout = 1 };
+inline int sm_count() { return 148; }
 inline uint8_t smem[232448] __attribute__((aligned(1024)));       // dynamic shared memory, by the
 inline uint8_t smem_raw[232448] __attribute__((aligned(1024)));   // names the kernels give it
 inline uint8_t ring[232448] __attribute__((aligned(1024)));
