@@ -11,6 +11,8 @@
 
 namespace mb200 {
 
+int sm_count();
+
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z),
          d = unpack_bf16x2(u.w);
@@ -334,7 +336,7 @@ static int launch_rmsnorm_bwd(int nb, const __nv_bfloat16* dy, const __nv_bfloat
                               __nv_bfloat16* dw, int dw_accumulate, int rows, int d, int* status,
                               cudaStream_t st) {
   int rc;
-  const int resident = d > 4096 ? 148 : d > 2048 ? 296 : 592;
+  const int resident = sm_count() * (d > 4096 ? 1 : d > 2048 ? 2 : 4);
   if (nb > resident) nb = resident;
 #define MB200_RMS_BWD(NT, NCH)                                                                  \
   (dres ? launch_rmsnorm_bwd_t<NT, NCH, true>(nb, dy, x, w, rstd, dres, dx, dw_partial, rows, d, \
@@ -747,7 +749,7 @@ extern "C" int mb200_rmsnorm_fwd(const void* x, const void* w, void* y, float* r
 }
 
 extern "C" int mb200_rmsnorm_bwd_blocks(int rows) {
-  const int cap = 148 * 4;   // one resident wave: four blocks per SM at d <= 2048
+  const int cap = sm_count() * 4;   // one resident wave: four blocks per SM at d <= 2048
   return rows < cap ? rows : cap;
 }
 
