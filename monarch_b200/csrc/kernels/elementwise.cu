@@ -60,19 +60,21 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 // ------------------------------------------------------------------ RMSNorm --
 // A row is held in registers by WPR warps (16-byte loads, NV per lane, all in flight at once)
-// and read from memory once; with one warp per row there is no block barrier at all.  Eight
-// loads per lane: with 16 (one warp per 4096 columns) too few warps fit, 33.6 us.  Bound by
-// HBM: 8192x4096 29.5 -> 26.4 us (134 MB), 8192x5120 37.6 -> 31.6 us.
+// and read from memory once; with one warp per row there is no block barrier at all.  Bound by
+// HBM for many rows, by the chain of a row's loads, reduction and stores for few: then more warps
+// with fewer loads each are faster (rmsnorm_fwd below has both sides).
+constexpr int rms_fwd_threads(int wpr) { return wpr > 4 ? 32 * wpr : 128; }
 template <int NV, int WPR>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(rms_fwd_threads(WPR))
     rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x,
                            const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                            float* __restrict__ rstd, int rows, int d, float eps) {
   dep_wait();
-  __shared__ float red[4];
+  constexpr int kRows = rms_fwd_threads(WPR) / 32 / WPR;   // of a block
+  __shared__ float red[kRows * WPR];
   const int warp = threadIdx.x >> 5;
   const int t = (int)threadIdx.x % (32 * WPR);   // place in the row's group of warps
-  const int row = (int)blockIdx.x * (4 / WPR) + warp / WPR;
+  const int row = (int)blockIdx.x * kRows + warp / WPR;
   const bool on = row < rows;
   const __nv_bfloat16* xr = x + (size_t)row * d;
   uint4 v[NV];
@@ -735,14 +737,31 @@ extern "C" int mb200_rmsnorm_fwd(const void* x, const void* w, void* y, float* r
                                  int d, float eps, void* stream) {
   if (rows <= 0) return 0;
   if (d % 8) return 1001;
-#define MB200_RMS_FWD(NV, WPR)                                                              \
-  return (int)launch_dep(rmsnorm_fwd_row_kernel<NV, WPR>, blocks_for(rows, 4 / WPR), 128, 0, \
-                         ST(stream), CBF(x), CBF(w), BF(y), rstd, rows, d, eps)
+#define MB200_RMS_FWD(NV, WPR)                                                           \
+  return (int)launch_dep(rmsnorm_fwd_row_kernel<NV, WPR>,                                 \
+                         blocks_for(rows, rms_fwd_threads(WPR) / 32 / WPR),               \
+                         rms_fwd_threads(WPR), 0, ST(stream), CBF(x), CBF(w), BF(y), rstd, rows, \
+                         d, eps)
+  // us on (loads per lane, warps per row); the limits lie between the measured row counts
+  //   d  512: 1000 rows (2,1) 1.85 (2,2) 1.70;   4000 rows 2.29 and 2.69
+  //   d 1024: 1000 rows (4,1) 2.48 (2,4) 1.96;   4000 rows 2.96 and 3.84
+  //   d 1032: 1000 rows (4,2) 2.48 (2,4) 2.29;   4000 rows (8,1) 5.03 (4,2) 4.17 (2,4) 4.18;
+  //           8192 rows 7.8, 8.0, 8.9
+  //   d 2048:   16 rows (8,1) 3.14 (2,4) 1.71;   8192 rows 13.25, (4,2) 12.30, 12.25
+  //   d 4096:   16 rows (8,2) 3.17 (4,4) 2.29 (2,8) 1.76;  1000 rows 4.02, 3.21, 3.56;
+  //           8192 rows 24.7, 23.0 (5.8 TB/s), 23.9
+  //   d 5120:   16 rows (8,4) 2.52 (4,8) 2.13;   8192 rows 29.9 and 30.9
+  //   d 8192:   16 rows (8,4) 3.15 (4,8) 2.39;   8192 rows 44.1 and 42.5
+  const bool few = rows <= 2048;
+  if (d <= 512 && few) MB200_RMS_FWD(2, 2);
   if (d <= 512) MB200_RMS_FWD(2, 1);
-  if (d <= 1024) MB200_RMS_FWD(4, 1);
-  if (d <= 2048) MB200_RMS_FWD(8, 1);
-  if (d <= 4096) MB200_RMS_FWD(8, 2);
-  if (d <= 8192) MB200_RMS_FWD(8, 4);
+  if (d <= 1024 && !few) MB200_RMS_FWD(4, 1);
+  if (d <= 2048 && !few) MB200_RMS_FWD(4, 2);
+  if (d <= 2048) MB200_RMS_FWD(2, 4);
+  if (d <= 4096 && rows <= 768) MB200_RMS_FWD(2, 8);
+  if (d <= 4096) MB200_RMS_FWD(4, 4);
+  if (d <= 6144 && !few) MB200_RMS_FWD(8, 4);
+  if (d <= 8192) MB200_RMS_FWD(4, 8);
 #undef MB200_RMS_FWD
   return (int)launch_dep(rmsnorm_fwd_kernel, rows, 256, 0, ST(stream), CBF(x), CBF(w), BF(y), rstd,
                          d, eps);
