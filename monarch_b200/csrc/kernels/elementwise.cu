@@ -358,22 +358,21 @@ static int launch_rmsnorm_bwd(int nb, const __nv_bfloat16* dy, const __nv_bfloat
 }
 
 // --------------------------------------------------------------------- RoPE --
-// Eight heads' worth of threads per row: a thread keeps the 8 cosines and sines of its column
-// pairs and applies them to every eighth head, ROPE_U heads at a time so that their loads are
-// in flight together.  (One thread per head and 8 pairs spent its time in 64-bit divisions and
-// in reading the tables again for every head: 8192 rows of 40 heads of 128 38.3 -> 31.1 us.)
+// A thread keeps the 8 cosines and sines of its column pairs and applies them to every step-th
+// head of its row, ROPE_U heads at a time so that their loads are in flight together.  (One
+// thread per head and 8 pairs spent its time in 64-bit divisions and in reading the tables again
+// for every head: 8192 rows of 40 heads of 128 32.1 us, so 27.1.)
 constexpr int ROPE_U = 5;
 __global__ void __launch_bounds__(256)
     rope_row_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                     const float* __restrict__ sin_t, int rows, int seq_len, int n_rot_heads,
-                    int log2_hd, int row_stride, int inverse) {
+                    int log2_hd, int log2_step, int row_stride, int inverse) {
   dep_wait();
-  const int hd = 1 << log2_hd, half = hd >> 1, per_head = hd >> 4;
-  const int log2_row = log2_hd - 1;   // hd / 2 = 8 * per_head threads per row
+  const int hd = 1 << log2_hd, half = hd >> 1, per_head = hd >> 4, step = 1 << log2_step;
+  const int log2_row = log2_hd - 4 + log2_step;   // step * per_head threads per row
   const int row = ((int)blockIdx.x << (8 - log2_row)) + ((int)threadIdx.x >> log2_row);
   if (row >= rows) return;
-  const int t = (int)threadIdx.x & (half - 1);
-  constexpr int step = 8;
+  const int t = (int)threadIdx.x & ((1 << log2_row) - 1);
   const int j = t & (per_head - 1);
   const size_t tab = (size_t)(row % seq_len) * half + j * 8;
   float c[8], s[8];
@@ -416,6 +415,23 @@ __global__ void __launch_bounds__(256)
       }
     }
   }
+}
+
+// log2 of `step`, the heads that a row's threads work on side by side (at most 256 threads).
+// Many rows: up to 8 heads per thread, so that the tables are read by few, and no more than 8 side
+// by side.  Few rows: 64 Ki threads if there are that many pairs of columns, since a thread's
+// batches follow one another.  us by step, heads of 128:
+//   8192 rows,  1 head 1: 2.2, 8: 8.7;   8 heads 1: 4.6, 2: 4.9, 8: 9.6;   20 heads 2: 15.0,
+//               4: 14.7, 8: 18.1;   40 heads 4: 27.7, 8: 27.1, 16: 34.2;   80 heads 4: 54.0,
+//               8: 52.2, 16: 54.3
+//   2048 rows, 20 heads 2: 3.5, 4: 3.3, 8: 4.1;   512 rows, 20 heads 4: 2.4, 8: 2.1, 32: 3.2
+//     64 rows, 40 heads 8: 2.3, 32: 1.9;   heads of 64: 80 heads 8: 3.9, 64: 1.8
+static inline int rope_log2_step(int rows, int heads, int log2_hd) {
+  const int most = 12 - log2_hd;
+  int s = 0;
+  while (s < most && s < 3 && (8 << s) < heads) ++s;
+  while (s < most && (1 << s) < heads && ((long long)rows << (s + log2_hd - 3)) <= 64 * 1024) ++s;
+  return s;
 }
 
 // Head sizes that are no power of two up to 512.
@@ -789,9 +805,11 @@ extern "C" int mb200_rope_inplace(void* qkv, const float* cos_t, const float* si
   if (rows <= 0) return 0;
   if (hd % 16 || row_stride % 8 || hd <= 0 || n_rot_heads <= 0) return 1001;
   if (hd <= 512 && (hd & (hd - 1)) == 0 && aligned16(cos_t) && aligned16(sin_t)) {
-    return (int)launch_dep(rope_row_kernel, blocks_for(rows, 32 / (hd / 16)), 256, 0, ST(stream),
-                           BF(qkv), cos_t, sin_t, rows, seq_len, n_rot_heads, __builtin_ctz(hd),
-                           row_stride, inverse);
+    const int log2_hd = __builtin_ctz(hd);
+    const int log2_step = rope_log2_step(rows, n_rot_heads, log2_hd);
+    return (int)launch_dep(rope_row_kernel, blocks_for(rows, 256 >> (log2_hd - 4 + log2_step)), 256,
+                           0, ST(stream), BF(qkv), cos_t, sin_t, rows, seq_len, n_rot_heads, log2_hd,
+                           log2_step, row_stride, inverse);
   }
   const long long total = (long long)rows * n_rot_heads * (hd / 16);
   return (int)launch_dep(rope_kernel, blocks_for(total, 256), 256, 0, ST(stream), BF(qkv), cos_t,
