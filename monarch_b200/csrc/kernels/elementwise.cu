@@ -471,13 +471,14 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
 
 // ------------------------------------------------------------------- SwiGLU --
 // Rows on grid.x, 8-column chunks on grid.y: no division per thread (a 64-bit one by F/8 cost
-// the forward a fifth of its time: 8192x14336 133.6 -> 113 us, backward 181 -> 178 us).
+// the forward a fifth of its time: 8192x14336 133.6 -> 113 us, backward 181 -> 178 us).  A block
+// takes several rows of fewer than 256 chunks.
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
-                                  __nv_bfloat16* __restrict__ h, int F) {
+                                  __nv_bfloat16* __restrict__ h, int rows, int F) {
   dep_wait();
-  const size_t row = blockIdx.x;
+  const size_t row = (size_t)blockIdx.x * blockDim.y + threadIdx.y;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (c >= F) return;
+  if (c >= F || row >= (size_t)rows) return;
   float g[8], u[8], o[8];
   load8(gu + row * 2 * F + c, g);
   load8(gu + row * 2 * F + F + c, u);
@@ -488,11 +489,11 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
 
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                   const __nv_bfloat16* __restrict__ dh,
-                                  __nv_bfloat16* __restrict__ dgu, int F) {
+                                  __nv_bfloat16* __restrict__ dgu, int rows, int F) {
   dep_wait();
-  const size_t row = blockIdx.x;
+  const size_t row = (size_t)blockIdx.x * blockDim.y + threadIdx.y;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (c >= F) return;
+  if (c >= F || row >= (size_t)rows) return;
   float g[8], u[8], d[8], dg[8], du[8];
   load8(gu + row * 2 * F + c, g);
   load8(gu + row * 2 * F + F + c, u);
@@ -507,8 +508,12 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
   store8(dgu + row * 2 * F + c, dg);
   store8(dgu + row * 2 * F + F + c, du);
 }
-// threads of a block and blocks along grid.y for rows of n 8-column chunks
-static inline int row_threads(int n) { return n >= 256 ? 256 : (n + 31) / 32 * 32; }
+// Block for rows of n 8-column chunks (x: chunks, y: rows), and the grid that covers them.  One
+// row per block, whatever its length, took 8192 rows of 64 columns 5.74 us, as long as rows of 512.
+static inline dim3 row_block(int n) { return n >= 256 ? dim3(256) : dim3(n, 256 / n); }
+static inline dim3 row_grid(int rows, int n, dim3 b) {
+  return dim3((rows + b.y - 1) / b.y, (n + b.x - 1) / b.x);
+}
 
 // ------------------------------------------------------------ cross-entropy --
 // One block per row; the row is read twice (maximum and sum, then the gradient) and written
@@ -697,11 +702,11 @@ __global__ void embedding_fwd_kernel(const __nv_bfloat16* __restrict__ table,
 // be): 8192x2048 34.8 -> 10.4 us against one pair per reduction.
 __global__ void embedding_bwd_vec_kernel(const __nv_bfloat16* __restrict__ dout,
                                          const int64_t* __restrict__ ids,
-                                         __nv_bfloat16* __restrict__ dtable, int d) {
+                                         __nv_bfloat16* __restrict__ dtable, int rows, int d) {
   dep_wait();
-  const size_t row = blockIdx.x;
+  const size_t row = (size_t)blockIdx.x * blockDim.y + threadIdx.y;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (c >= d) return;
+  if (c >= d || row >= (size_t)rows) return;
   const int64_t id = ids[row];
   const uint4 g = *reinterpret_cast<const uint4*>(dout + row * d + c);
   asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dtable + id * d + c),
@@ -819,17 +824,17 @@ extern "C" int mb200_rope_inplace(void* qkv, const float* cos_t, const float* si
 extern "C" int mb200_swiglu_fwd(const void* gu, void* h, int rows, int F, void* stream) {
   if (rows <= 0) return 0;
   if (F % 8 || F <= 0) return 1001;
-  const int nt = row_threads(F / 8);
-  return (int)launch_dep(swiglu_fwd_kernel, dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream),
-                         CBF(gu), BF(h), F);
+  const dim3 b = row_block(F / 8);
+  return (int)launch_dep(swiglu_fwd_kernel, row_grid(rows, F / 8, b), b, 0, ST(stream), CBF(gu),
+                         BF(h), rows, F);
 }
 extern "C" int mb200_swiglu_bwd(const void* gu, const void* dh, void* dgu, int rows, int F,
                                 void* stream) {
   if (rows <= 0) return 0;
   if (F % 8 || F <= 0) return 1001;
-  const int nt = row_threads(F / 8);
-  return (int)launch_dep(swiglu_bwd_kernel, dim3(rows, blocks_for(F / 8, nt)), nt, 0, ST(stream),
-                         CBF(gu), CBF(dh), BF(dgu), F);
+  const dim3 b = row_block(F / 8);
+  return (int)launch_dep(swiglu_bwd_kernel, row_grid(rows, F / 8, b), b, 0, ST(stream), CBF(gu),
+                         CBF(dh), BF(dgu), rows, F);
 }
 
 extern "C" int mb200_cross_entropy_fwd_bwd(void* logits, const int64_t* targets, float* loss_rows,
@@ -871,9 +876,9 @@ extern "C" int mb200_embedding_bwd(const void* dout, const int64_t* ids, void* d
   if (rows <= 0) return 0;
   if (d % 2 || d <= 0) return 1001;
   if (d % 8 == 0 && aligned16(dout) && aligned16(dtable)) {
-    const int nt = row_threads(d / 8);
-    return (int)launch_dep(embedding_bwd_vec_kernel, dim3(rows, blocks_for(d / 8, nt)), nt, 0,
-                           ST(stream), CBF(dout), ids, BF(dtable), d);
+    const dim3 b = row_block(d / 8);
+    return (int)launch_dep(embedding_bwd_vec_kernel, row_grid(rows, d / 8, b), b, 0, ST(stream),
+                           CBF(dout), ids, BF(dtable), rows, d);
   }
   const long long total = (long long)rows * (d / 2);
   return (int)launch_dep(embedding_bwd_kernel, blocks_for(total, 256), 256, 0, ST(stream),
