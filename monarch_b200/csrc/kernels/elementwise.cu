@@ -520,7 +520,14 @@ static inline dim3 row_grid(int rows, int n, dim3 b) {
 // once.  Bound by HBM and, close behind, by instructions (two exponentials per logit), hence the
 // two-wide arithmetic.  Long rows get blocks of 1024 threads: with two of them per SM most of
 // the rows being worked on (296 x 256 KB at a vocabulary of 128256) are still in L2 at their
-// second read, with four blocks of 512 they were not: 4096x128256 492 -> 390 us.
+// second read, with four blocks of 512 they were not: 4096x128256 492 -> 390 us.  Short rows get
+// small blocks, whose reductions and start-up are shorter.  us by threads of a block, 4096 rows:
+//   V  4096  128: 13.8  256: 17.6  512: 22.7      V 16384  128: 52.9  256: 46.9  512: 49.5
+//   V  6144  128: 21.5  256: 24.9  512: 30.9      V 32000  256: 101.7  512: 91.4  1024: 110.8
+//   V  8192  128: 26.7  256: 25.4  512: 35.9      V 50264  256: 188.9  512: 147.3  1024: 160.9
+//                                                 V 65536  256: 243.3  512: 206.0  1024: 182.8
+// Below 512 rows the chip is not full and a row's own time counts: 64 rows, V 4096 128: 2.9
+// 512: 2.7; V 6144 128: 3.6 512: 3.2; V 16384 256: 4.2 512: 3.8; V 65536 512: 8.0 1024: 7.8.
 template <int CE_THREADS>
 __global__ void __launch_bounds__(CE_THREADS, 2048 / CE_THREADS)
     cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
@@ -845,8 +852,10 @@ extern "C" int mb200_cross_entropy_fwd_bwd(void* logits, const int64_t* targets,
 #define MB200_CE(NT)                                                                      \
   return (int)launch_dep(cross_entropy_kernel<NT>, rows, NT, 0, ST(stream), BF(logits), targets, \
                          loss_rows, V, ld, grad_scale)
-  if (V <= 4096) MB200_CE(128);
-  if (V <= 65536) MB200_CE(512);
+  const bool many = rows >= 512;
+  if (V <= (many ? 6144 : 4096)) MB200_CE(128);
+  if (many && V <= 16384) MB200_CE(256);
+  if (V < 65536) MB200_CE(512);
   MB200_CE(1024);
 #undef MB200_CE
 }
