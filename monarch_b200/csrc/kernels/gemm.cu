@@ -417,14 +417,25 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams&
 static int g_gemm_impl = 2;
 
 // Tile and K split of the plain product under implementation 2: the smallest estimate of
-//   t0 + waves * (64-deep steps of one CTA or pair) * c
+//   t0 + (waves - 1) * max(steps * c, e) + steps * c,   steps: 64-deep steps of one CTA or pair
 // with the microseconds measured on this chip.  c is what limits a step: 32 KB per SM and the
-// tensor pipe for the pair, the 24 to 48 KB that one SM fetches for the others.  t0 is launch,
-// first load, last epilogue; a split adds its cluster barriers and the exchange.  Estimate ->
+// tensor pipe for the pair, the 24 to 48 KB that one SM fetches for the others.  e is a tile's
+// epilogue, which a further wave hides behind its products or waits for; t0 is launch, first
+// load, last epilogue; a split adds its cluster barriers and the exchange.  Estimate ->
 // measured, us: 8192x1024x1024 pair 18.0 -> 18.1; 2048x4096x4096 pair 51.2 -> 50.2, 128x256
-// 54.5 -> 55.1, 128x128 67.0 -> 68.7; 2048^3 128x256 17.5 -> 16.9, pair 18.0 -> 18.6;
-// 1000x2048x3072 128x128 16.1 -> 15.0, pair 23.6 -> 20.5; 200x768x256 128x64 4.4 -> 4.7, pair
-// 8.4 -> 9.0; 64x4096x4096 128x128 in 4 parts 10.3 -> 10.1, 128x64 in 2 parts 10.8 -> 11.1.
+// 54.5 -> 55.1, 128x128 67.0 -> 68.7; 2048^3 128x256 17.5 -> 15.2, pair 18.0 -> 16.6;
+// 1000x2048x3072 128x128 16.1 -> 14.4, pair 23.6 -> 21.2; 200x768x256 128x64 4.4 -> 4.7, pair
+// 8.4 -> 9.0; 64x4096x4096 128x128 in 4 parts 10.3 -> 10.1, 128x64 in 2 parts 10.8 -> 11.1;
+// 1704x13136x160 pair 29.2 -> 27.8, 128x256 28.5 -> 23.2.
+//
+// Rows of A, B or C that do not start on 128-byte lines cost the single CTAs more than the pair,
+// whose tiles share fewer lines with their neighbours: kUnaligned, for 128x256 always, for the
+// narrower ones once there is more than one wave.  2944x408x5432 128x256 53.4 us, pair 41.3;
+// 352x13448x1352 128x128 31.7 and 28.8; 6968x984x912 27.1 and 24.6; but 3072x2048x1000 with both
+// operands along 3072 and 2048 128x128 15.8 and 17.8.  Over 44 shapes in four layouts the choice
+// takes 0.8 % more than the best tile; without e and kUnaligned 3.4 %, and 26 of the 144
+// products that no split takes were slower than the pair, by up to 17 %.
+constexpr float kUnaligned = 1.15f;
 struct GemmPlan {
   int bn;      // 0: the CTA pair's 256x256 tile, else the columns of a single CTA's 128-row tile
   int split;   // CTAs of a cluster that share a tile along K
@@ -439,20 +450,27 @@ static int split_clusters(int bn, int split) {
          : split == 4 ? split_capacity<false, false, 128, 4>()
                       : split_capacity<false, false, 128, 8>();
 }
-static GemmPlan gemm_plan(int M, int N, int K) {
+// aligned: the leading dimensions of A, B and C are multiples of 64 elements
+static GemmPlan gemm_plan(int M, int N, int K, bool aligned) {
   const int iters = (K + GEMM_BK - 1) / GEMM_BK;
   const auto div = [](long long a, long long b) { return (a + b - 1) / b; };
   const int sms = sm_count();
   GemmPlan best = {0, 1};
-  float t = 7.0f + 0.345f * iters * div(div(M, G2_BM) * div(N, G2_BN), sms / 2);
-  struct { int bn; float t0, c, t_split[3]; } const kinds[] = {
-      {256, 5.2f, 0.385f, {0.f, 0.f, 0.f}},
-      {128, 4.3f, 0.245f, {1.05f, 2.1f, 3.2f}},   // splits of 2, 4, 8
-      {64, 3.6f, 0.200f, {0.8f, 1.5f, 2.3f}},
+  const auto estimate = [&](float t0, float c, float e, long long waves) {
+    const float step = c * iters;
+    return t0 + (waves - 1) * (step > e ? step : e) + step;
+  };
+  float t = 0.98f * estimate(7.0f, 0.345f, 5.3f, div(div(M, G2_BM) * div(N, G2_BN), sms / 2));
+  struct { int bn; float t0, c, e, t_split[3]; } const kinds[] = {
+      {256, 5.2f, 0.385f, 4.6f, {0.f, 0.f, 0.f}},
+      {128, 4.3f, 0.245f, 3.0f, {1.05f, 2.1f, 3.2f}},   // splits of 2, 4, 8
+      {64, 3.6f, 0.200f, 2.2f, {0.8f, 1.5f, 2.3f}},
   };
   for (const auto& k : kinds) {
     const long long tiles = div(M, GEMM_BM) * div(N, k.bn);
-    const float u = k.t0 + k.c * iters * div(tiles, sms);
+    // an estimate within 2 % of the pair's goes to the pair (6136x5992x656 66.9, 128x256 83.4 us)
+    const float u = estimate(k.t0, k.c, k.e, div(tiles, sms)) *
+                    (aligned || (k.bn != 256 && tiles <= sms) ? 1.f : kUnaligned);
     if (u < t) t = u, best = {k.bn, 1};
     if (k.bn == 256) continue;
     for (int i = 0; i < 3; ++i) {
@@ -489,7 +507,8 @@ extern "C" int mb200_gemm_bf16(const void* A, const void* B, void* C, const void
   p.n_blk_rot = 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CUtensorMap ta, tb;
-  const GemmPlan plan = g_gemm_impl == 2 ? gemm_plan(M, N, K) : GemmPlan{GEMM_BN, 1};
+  const GemmPlan plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, ((lda | ldb | ldc) & 63) == 0)
+                                         : GemmPlan{GEMM_BN, 1};
   const int bn = plan.bn;
   if (bn == 0) {
     const int r = make_gemm2_tmaps(&ta, &tb, A, B, M, N, K, lda, ldb, a_mn, b_mn);
@@ -526,7 +545,7 @@ constexpr int kGluFwdMinK = 0, kGluFwdKeepMinK = 2560, kGluBwdMinK = 3072;
 
 // 1: CTA-pair tile, 0: small single-CTA tile, -1: two kernels are faster (or only they can).
 static int glu_tile(int M, int N, int F, int K, int min_k, GemmPlan* plan) {
-  *plan = g_gemm_impl == 2 ? gemm_plan(M, N, K) : GemmPlan{128, 1};
+  *plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, true) : GemmPlan{128, 1};
   if (plan->split > 1) return -1;
   if (plan->bn != 0 && plan->bn != 256) return 0;
   return F % 128 == 0 && K >= min_k ? 1 : -1;
@@ -599,6 +618,15 @@ extern "C" int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* g
   const int grid = tiles < sm_count() ? tiles : sm_count();
   return plan.bn == 64 ? launch<false, true, 64, kEpiSwigluBwd>(ta, tb, p, grid, st)
                        : launch<false, true, 128, kEpiSwigluBwd>(ta, tb, p, grid, st);
+}
+
+// The tile (columns; 0: the CTA pair's) and K split that a product takes.
+extern "C" int mb200_gemm_plan(int M, int N, int K, int lda, int ldb, int ldc, int* bn, int* split) {
+  if (M <= 0 || N <= 0 || K <= 0) return 1001;
+  const GemmPlan plan = gemm_plan(M, N, K, ((lda | ldb | ldc) & 63) == 0);
+  *bn = plan.bn;
+  *split = plan.split;
+  return 0;
 }
 
 extern "C" int mb200_gemm_set_impl(int impl) {

@@ -24,8 +24,13 @@ int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void* gu, int M
 int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* gu, void* dgu, int M, int F,
                           int K, int lda, int ldw, int ld_gu, int* status, void* stream);
 
+// Tile and K split that implementation 2 takes for a product: columns of a single CTA's 128-row
+// tile (0: 256x256 of a CTA pair) and CTAs that share it along K.
+int mb200_gemm_plan(int M, int N, int K, int lda, int ldb, int ldc, int* bn, int* split);
+
 // Which GEMM kernel the library uses: 1 = single-CTA 128x256 tiles, 2 = CTA-pair 256x256
-// tiles, or smaller ones for products with few tiles (default).  The fused collective+GEMM kernels follow the same setting.
+// tiles, or smaller ones for products with few tiles (default).  The fused collective+GEMM
+// kernels follow the same setting.
 int mb200_gemm_set_impl(int impl);
 int mb200_gemm_get_impl(void);
 

@@ -85,6 +85,7 @@ def _declare(l: ctypes.CDLL) -> None:
 _OPTIONAL: dict[str, list] = {
     "mb200_gemm_swiglu_fwd": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "mb200_gemm_swiglu_bwd": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "mb200_gemm_plan": [_i, _i, _i, _i, _i, _i, _vp, _vp],
     "mb200_attn_fwd": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp],
     "mb200_attn_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                        _i, _i, _f, _vp, _vp],
@@ -156,6 +157,16 @@ def bounds_register(ptr: int, nbytes: int, device=None) -> None:
             check(l.mb200_bounds_reset(status_word(idx).data_ptr()), "bounds_reset", 0)
             _bounds_ready.add(idx)
         check(l.mb200_bounds_register(ptr, nbytes), "bounds_register", 0)
+
+
+def gemm_plan(M: int, N: int, Kd: int, lda: int, ldb: int, ldc: int) -> tuple:
+    """(columns of the tile, CTAs that share it along K) of a product under implementation 2;
+    0 columns stand for the CTA pair's 256x256 tile."""
+    bn, split = ctypes.c_int(), ctypes.c_int()
+    rc = lib().mb200_gemm_plan(M, N, Kd, lda, ldb, ldc, ctypes.byref(bn), ctypes.byref(split))
+    if rc:
+        raise KernelError(f"no plan for a {M}x{N}x{Kd} product")
+    return bn.value, split.value
 
 
 def set_gemm_impl(impl: int) -> None:

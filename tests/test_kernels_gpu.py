@@ -223,11 +223,21 @@ def test_optimizer_overlapped_with_backward_is_bit_identical():
 
 
 # (M, N, K): what each tile of the plain product covers -- 128x64 and its splits (few rows, long
-# K; fewer rows and columns than a tile; remainders in M, N and K), 128x128 and its splits,
-# 128x256, and one row
-@pytest.mark.parametrize("M,N,K_", [(200, 768, 256), (1, 264, 4096), (64, 512, 4104), (96, 4096, 4096),
-                                    (8, 24, 1032), (333, 1496, 1096), (1000, 2048, 1544),
-                                    (257, 6144, 1024), (2048, 2048, 2056)])
+# K; fewer rows and columns than a tile; remainders in M, N and K), 128x128 and its splits in 2, 4
+# and 8 parts, 128x256, the CTA pair, one row, and a K beyond 20000
+GEMM_SHAPES = [(200, 768, 256), (1, 264, 4096), (64, 512, 4104), (96, 4096, 4096), (8, 24, 1032),
+               (333, 1496, 1096), (1000, 2048, 1544), (257, 6144, 1024), (2048, 2048, 2056),
+               (8, 8200, 2056), (24, 1496, 8200), (100, 1032, 20008), (2040, 4104, 1096),
+               (250, 12008, 264)]
+
+
+def test_gemm_shapes_reach_every_tile_and_split():
+    plans = {K.gemm_plan(M, N, K_, K_, K_, N + 8) for M, N, K_ in GEMM_SHAPES}
+    assert plans == {(0, 1), (256, 1), (128, 1), (128, 2), (128, 4), (128, 8), (64, 1), (64, 2),
+                     (64, 4), (64, 8)}
+
+
+@pytest.mark.parametrize("M,N,K_", GEMM_SHAPES)
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
 def test_gemm_tile_choice(M, N, K_, a_mn, b_mn):
     """Every tile and split the product can choose, against 64 bits: the only rounding is that
