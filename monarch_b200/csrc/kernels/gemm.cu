@@ -531,36 +531,71 @@ extern "C" int mb200_gemm_bf16(const void* A, const void* B, void* C, const void
 // two products.  The gate and up columns of an output column meet in one tile because its B rows
 // come from both halves of W.
 //
-// What it saves is the pass over memory (and for small products the launch); what it costs is a
-// longer epilogue, which the next tile's products hide if K is long enough.  Product plus
-// activation as two kernels -> as one, us, the two timed in turn:
-//   forward without gu   T 8192 F 14336 K 4096 1528 -> 1351, K 2048 F 8192 503 -> 409,
-//                        K 1024 F 4096 200 -> 164, K 512 F 8192 349 -> 296
-//   forward with gu      T 8192 F 14336 K 4096 1528 -> 1393, K 2560 F 4096 256 -> 245,
-//                        K 2048 F 8192 503 -> 540 (two kernels there)
-//   backward             T 8192 F 14336 K 4096 978 -> 855, K 3072 F 8192 454 -> 433,
-//                        K 2560 F 4096 189 -> 197 (two kernels there)
-//   256x512x256 on small tiles 22.0 -> 14.7 and 21.5 -> 13.9 with the host's part.
-constexpr int kGluFwdMinK = 0, kGluFwdKeepMinK = 2560, kGluBwdMinK = 3072;
+// What it saves is the pass over memory and a launch; what it costs is a longer epilogue, which
+// the next tile's products hide if there is a next one and K is long enough.  Device time of the
+// two kernels -> of one, us (T rows, both in turn, w of 0.02):
+//   pair tiles, forward without gu: faster wherever the pair is the product's own tile: T 8192
+//     F 14336 K 4096 1348 -> 1186, K 512 428 -> 321, T 2048 F 2048 K 3072 42 -> 40.  Where the
+//     product alone would take 128x256 tiles the pair's loss comes first: T 1024 F 2048 K 2048
+//     18.9 -> 19.5, T 2048 F 8192 K 256 (7 waves of pairs) 50.2 -> 50.4, T 4096 F 8192 K 256
+//     (14 waves) 110 -> 100.
+//   pair tiles, forward with gu: T 8192 F 14336 K 4096 1348 -> 1271, F 2048 K 2560 129 -> 123,
+//     K 2048 108 -> 107; T 4096 F 2048 K 2560 70 -> 68, F 1024 37.0 -> 38.3, F 4096 K 2048
+//     109 -> 113; T 2048 F 8192 K 3072 151 -> 154.
+//   pair tiles, backward: T 8192 F 14336 K 4096 988 -> 888, F 2048 K 4096 121 -> 115, K 3072
+//     97.2 -> 97.6, K 2560 93 -> 98; T 2048 F 4096 K 4096 61.4 -> 61.0, F 2048 (one wave)
+//     34.2 -> 36.9.
+//   small tiles: always slower on the device (256x512x256 6.2 -> 8.4 forward and 6.4 -> 8.4
+//     backward; 8192x2048x256 backward 53 -> 97), but with one wave by no more than the second
+//     launch costs the host, which is what calls as short as that wait for.  128x128 tiles lose
+//     4.4 us in the backward.
+constexpr int kGluKeepMinK = 2560, kGluKeepMinM = 4096, kGluKeepMinTiles = 256;
+constexpr int kGluBwdMinK = 4096;
+constexpr int kGluSmallMaxK = 1024;   // longer products outlast the host's second launch
 
-// 1: CTA-pair tile, 0: small single-CTA tile, -1: two kernels are faster (or only they can).
-static int glu_tile(int M, int N, int F, int K, int min_k, GemmPlan* plan) {
-  *plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, true) : GemmPlan{128, 1};
+enum GluKind { kGluFwd, kGluFwdKeep, kGluBwd };
+// 1: CTA-pair tile, 0: small single-CTA tile, -1: two kernels.
+static int glu_tile(GluKind kind, int M, int N, int F, int K, bool aligned, GemmPlan* plan) {
+  *plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, aligned) : GemmPlan{128, 1};
   if (plan->split > 1) return -1;
-  if (plan->bn != 0 && plan->bn != 256) return 0;
-  return F % 128 == 0 && K >= min_k ? 1 : -1;
+  const auto div = [](int a, int b) { return (long long)(a + b - 1) / b; };
+  if (plan->bn == 64 || plan->bn == 128) {
+    if (kind == kGluBwd && plan->bn != 64) return -1;
+    return div(M, GEMM_BM) * div(F, 64) <= sm_count() && K <= kGluSmallMaxK ? 0 : -1;
+  }
+  if (F % 128) return -1;
+  const long long tiles = div(M, G2_BM) * div(N, G2_BN), pairs = sm_count() / 2;
+  bool fuse;
+  if (kind == kGluFwd)
+    fuse = plan->bn == 0 || tiles > 8 * pairs;
+  else if (kind == kGluFwdKeep)
+    fuse = plan->bn == 0 && K >= kGluKeepMinK && M >= kGluKeepMinM && tiles >= kGluKeepMinTiles;
+  else
+    fuse = plan->bn == 0 && K >= kGluBwdMinK && tiles > pairs;
+  return fuse ? 1 : -1;
 }
 
 extern "C" int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void* gu, int M, int F,
-                                     int K, int lda, int ldw, int ldh, int ld_gu, int* status,
-                                     void* stream) {
+                                     int K, int lda, int ldw, int ldh, int ld_gu, int keep_gu,
+                                     int* status, void* stream) {
   if (M <= 0 || F <= 0 || K <= 0) return 0;
-  if (F % 64 || (ldh & 7) || (ld_gu & 7) || ((reinterpret_cast<uintptr_t>(H) |
-                                              reinterpret_cast<uintptr_t>(gu)) & 15))
+  if (F % 64 || (ldh & 7) || (ld_gu & 7) || (keep_gu && !gu) ||
+      ((reinterpret_cast<uintptr_t>(H) | reinterpret_cast<uintptr_t>(gu)) & 15))
     return 1001;
   GemmPlan plan;
-  const int tile = glu_tile(M, 2 * F, F, K, gu ? kGluFwdKeepMinK : kGluFwdMinK, &plan);
-  if (tile < 0) return MB200_NOT_FUSED;
+  const int tile = glu_tile(keep_gu ? kGluFwdKeep : kGluFwd, M, 2 * F, F, K,
+                            ((lda | ldw | ldh | ld_gu) & 63) == 0, &plan);
+  if (tile < 0) {
+    if (!gu) return MB200_NOT_FUSED;
+    const int rc = ld_gu == 2 * F && ldh == F
+                       ? mb200_gemm_bf16(A, W, gu, nullptr, M, 2 * F, K, lda, ldw, ld_gu, 0, 0, 0, 0,
+                                         status, stream)
+                       : 1001;
+    if (rc) return rc;
+    const int rc2 = mb200_swiglu_fwd(gu, H, M, F, stream);
+    return rc2 ? rc2 : MB200_TWO_KERNELS;
+  }
+  if (!keep_gu) gu = nullptr;
   GemmParams p{};
   p.C = reinterpret_cast<__nv_bfloat16*>(H);
   p.M = M; p.N = 2 * F; p.K = K;
@@ -588,16 +623,24 @@ extern "C" int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void
 
 // dgu[M, 2F] = gradient of silu(gate) * up at gu for dh = A W (W [K, F] row-major), without
 // storing dh.
-extern "C" int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* gu, void* dgu, int M,
-                                     int F, int K, int lda, int ldw, int ld_gu, int* status,
-                                     void* stream) {
+extern "C" int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* gu, void* dgu,
+                                     void* dh, int M, int F, int K, int lda, int ldw, int ld_gu,
+                                     int* status, void* stream) {
   if (M <= 0 || F <= 0 || K <= 0) return 0;
   if (F % 32 || (ld_gu & 7) || ((reinterpret_cast<uintptr_t>(gu) |
                                  reinterpret_cast<uintptr_t>(dgu)) & 15))
     return 1001;
   GemmPlan plan;
-  const int tile = glu_tile(M, F, F, K, kGluBwdMinK, &plan);
-  if (tile < 0) return MB200_NOT_FUSED;
+  const int tile = glu_tile(kGluBwd, M, F, F, K, ((lda | ldw | ld_gu) & 63) == 0, &plan);
+  if (tile < 0) {
+    if (!dh) return MB200_NOT_FUSED;
+    const int rc = ld_gu == 2 * F ? mb200_gemm_bf16(A, W, dh, nullptr, M, F, K, lda, ldw, F, 0, 0, 1, 0,
+                                                    status, stream)
+                                  : 1001;
+    if (rc) return rc;
+    const int rc2 = mb200_swiglu_bwd(gu, dh, dgu, M, F, stream);
+    return rc2 ? rc2 : MB200_TWO_KERNELS;
+  }
   GemmParams p{};
   p.M = M; p.N = F; p.K = K;
   p.status = status;
@@ -612,12 +655,11 @@ extern "C" int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* g
     const int r = make_gemm2_tmaps(&ta, &tb, A, W, M, F, K, lda, ldw, 0, 1);
     return r ? 1000 - r : launch2<false, true, kEpiSwigluBwd>(ta, tb, p, st);
   }
-  const int r = make_gemm_tmaps_bn(&ta, &tb, A, W, M, F, K, lda, ldw, 0, 1, plan.bn);
+  const int r = make_gemm_tmaps_bn(&ta, &tb, A, W, M, F, K, lda, ldw, 0, 1, 64);
   if (r) return 1000 - r;
-  const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((F + plan.bn - 1) / plan.bn);
+  const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((F + 63) / 64);
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  return plan.bn == 64 ? launch<false, true, 64, kEpiSwigluBwd>(ta, tb, p, grid, st)
-                       : launch<false, true, 128, kEpiSwigluBwd>(ta, tb, p, grid, st);
+  return launch<false, true, 64, kEpiSwigluBwd>(ta, tb, p, grid, st);
 }
 
 // The tile (columns; 0: the CTA pair's) and K split that a product takes.

@@ -14,15 +14,18 @@ int mb200_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M,
                     int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int accumulate,
                     int* status, void* stream);
 
-// H[M,F] = silu(A Wg^T) * (A Wu^T), W = [Wg; Wu] row-major [2F,K]; gu ([M,2F], may be null)
-// receives the two products.  F % 64 == 0.  Both functions return MB200_NOT_FUSED, and launch
-// nothing, for products that are faster as two kernels.
+// H[M,F] = silu(A Wg^T) * (A Wu^T), W = [Wg; Wu] row-major [2F,K]; with keep_gu gu ([M,2F])
+// receives the two products.  F % 64 == 0.  Both functions launch two kernels, and return
+// MB200_TWO_KERNELS, where that is faster; these need the matrix between them (gu here, dh [M,F]
+// below, both contiguous), and where it is null they return MB200_NOT_FUSED and launch nothing.
 #define MB200_NOT_FUSED 1003
+#define MB200_TWO_KERNELS 1004
 int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void* gu, int M, int F, int K,
-                          int lda, int ldw, int ldh, int ld_gu, int* status, void* stream);
+                          int lda, int ldw, int ldh, int ld_gu, int keep_gu, int* status,
+                          void* stream);
 // dgu[M,2F] = gradient of silu(gate)*up at gu for dh = A W, W row-major [K,F].  F % 32 == 0.
-int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* gu, void* dgu, int M, int F,
-                          int K, int lda, int ldw, int ld_gu, int* status, void* stream);
+int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* gu, void* dgu, void* dh, int M,
+                          int F, int K, int lda, int ldw, int ld_gu, int* status, void* stream);
 
 // Tile and K split that implementation 2 takes for a product: columns of a single CTA's 128-row
 // tile (0: 256x256 of a CTA pair) and CTAs that share it along K.

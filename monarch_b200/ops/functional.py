@@ -145,7 +145,11 @@ def swiglu_bwd(gu, dh, out=None):
     return dgu
 
 
-_NOT_FUSED = 1003   # MB200_NOT_FUSED: this product is faster as two kernels
+_NOT_FUSED, _TWO_KERNELS = 1003, 1004   # MB200_NOT_FUSED, MB200_TWO_KERNELS
+
+
+def _check_glu(rc, what):
+    K.check(0 if rc == _TWO_KERNELS else rc, what, 2 if rc == _TWO_KERNELS else 1)
 
 
 def gemm_swiglu(a, w_gu, keep_gu=True):
@@ -159,15 +163,15 @@ def gemm_swiglu(a, w_gu, keep_gu=True):
         assert w_gu.shape == (2 * F, Kd), (a.shape, w_gu.shape)
         h = torch.empty(T, F, dtype=bf16, device=a.device)
         gu = torch.empty(T, 2 * F, dtype=bf16, device=a.device) if keep_gu else None
-        rc = K.lib().mb200_gemm_swiglu_fwd(
-            a.data_ptr(), w_gu.data_ptr(), h.data_ptr(), _p(gu), T, F, Kd, lda, ldw, F, 2 * F,
-            K.status_ptr(a), K.stream_ptr())
-        if rc != _NOT_FUSED:
-            K.check(rc, "gemm_swiglu_fwd")
-            return h, gu
-        if keep_gu:
-            return swiglu_fwd(gemm(a, w_gu, out=gu), out=h), gu
-        return swiglu_fwd(gemm(a, w_gu), out=h), None
+        while True:
+            rc = K.lib().mb200_gemm_swiglu_fwd(
+                a.data_ptr(), w_gu.data_ptr(), h.data_ptr(), _p(gu), T, F, Kd, lda, ldw, F, 2 * F,
+                int(keep_gu), K.status_ptr(a), K.stream_ptr())
+            if rc != _NOT_FUSED:
+                break
+            gu = torch.empty(T, 2 * F, dtype=bf16, device=a.device)
+        _check_glu(rc, "gemm_swiglu_fwd")
+        return h, (gu if keep_gu else None)
     gu = gemm(a, w_gu)
     return swiglu_fwd(gu), (gu if keep_gu else None)
 
@@ -183,13 +187,16 @@ def gemm_swiglu_bwd(dy, w_down, gu):
         Kd = dy.shape[1]
         assert w_down.shape[0] == Kd and gu.shape == (T, 2 * F), (dy.shape, w_down.shape, gu.shape)
         dgu = torch.empty_like(gu)
-        rc = K.lib().mb200_gemm_swiglu_bwd(
-            dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, F, Kd, lda, ldw,
-            2 * F, K.status_ptr(dy), K.stream_ptr())
-        if rc != _NOT_FUSED:
-            K.check(rc, "gemm_swiglu_bwd")
-            return dgu
-        return swiglu_bwd(gu, gemm(dy, w_down, b_mn=True), out=dgu)
+        dh = None
+        while True:
+            rc = K.lib().mb200_gemm_swiglu_bwd(
+                dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(), _p(dh), T, F, Kd,
+                lda, ldw, 2 * F, K.status_ptr(dy), K.stream_ptr())
+            if rc != _NOT_FUSED:
+                break
+            dh = torch.empty(T, F, dtype=bf16, device=dy.device)
+        _check_glu(rc, "gemm_swiglu_bwd")
+        return dgu
     return swiglu_bwd(gu, gemm(dy, w_down, b_mn=True))
 
 

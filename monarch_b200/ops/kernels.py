@@ -83,8 +83,8 @@ def _declare(l: ctypes.CDLL) -> None:
 
 
 _OPTIONAL: dict[str, list] = {
-    "mb200_gemm_swiglu_fwd": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
-    "mb200_gemm_swiglu_bwd": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "mb200_gemm_swiglu_fwd": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "mb200_gemm_swiglu_bwd": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "mb200_gemm_plan": [_i, _i, _i, _i, _i, _i, _vp, _vp],
     "mb200_attn_fwd": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp],
     "mb200_attn_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,

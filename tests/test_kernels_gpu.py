@@ -347,27 +347,29 @@ def test_embedding_bwd_widths(d):
 
 
 # the fused tiles and their remainders in rows, K and (backward) F; F that takes the separate
-# kernels (200 % 64, 24 % 32), products split along K, pair tiles on both sides of the least K
+# kernels (200 % 64, 24 % 32), products split along K, more than one wave of small tiles and K too
+# long for them, pair tiles on both sides of the limits in K, in rows and in tiles
 @pytest.mark.parametrize("T,F,K_", [(1, 64, 64), (256, 512, 256), (200, 384, 136), (300, 96, 72),
                                     (130, 2048, 128), (77, 200, 64), (50, 24, 64), (64, 512, 4096),
-                                    (2049, 4096, 1024), (1100, 8192, 3080)])
+                                    (2049, 4096, 1024), (1100, 8192, 3080), (1030, 1024, 1088),
+                                    (4097, 512, 256), (4100, 2048, 2568), (4100, 2048, 4104),
+                                    (8200, 8192, 256)])
 def test_gemm_swiglu_equals_the_separate_kernels(gemm_impl, T, F, K_):
-    """The fused epilogues round where the separate kernels store, so the bits agree wherever
-    the product's own bits do (one K order); elsewhere within two bf16 roundings."""
+    """The fused epilogues round where the separate kernels store, and the products add along K in
+    the same order: the same bits."""
     torch.manual_seed(5)
     a = torch.randn(T, K_, device="cuda", dtype=bf16)
     w = (0.1 * torch.randn(2 * F, K_, device="cuda")).to(bf16)
     gu_ref = ops.gemm(a, w)
     h_ref = ops.swiglu_fwd(gu_ref)
     h, gu = ops.gemm_swiglu(a, w)
-    assert _rel(gu, gu_ref) < 1e-3 and _rel(h, h_ref) < 1e-3
-    assert torch.equal(ops.swiglu_fwd(gu), h)
+    assert torch.equal(gu, gu_ref) and torch.equal(h, h_ref)
     h2, none = ops.gemm_swiglu(a, w, keep_gu=False)
     assert none is None and torch.equal(h2, h)
     dy = torch.randn(T, K_, device="cuda", dtype=bf16)
     wd = (0.1 * torch.randn(K_, F, device="cuda")).to(bf16)
     ref = ops.swiglu_bwd(gu, ops.gemm(dy, wd, b_mn=True))
-    assert _rel(ops.gemm_swiglu_bwd(dy, wd, gu), ref) < 1e-3
+    assert torch.equal(ops.gemm_swiglu_bwd(dy, wd, gu), ref)
 
 
 def test_rmsnorm_bwd_on_two_streams_shares_no_scratch(monkeypatch):
