@@ -420,3 +420,63 @@ def test_checkpointing_keeps_the_residual_stream_only_when_asked(monkeypatch):
         grads[keep] = [g.clone() for u in range(cfg.n_layers + 2) for g in st.unit_grads(u).values()]
     assert held[True] - held[False] == cfg.n_layers * T * cfg.d * 2, held
     assert all(torch.equal(a, b) for a, b in zip(grads[False][1:], grads[True][1:]))
+
+
+# both sides of every limit in rows and width that the choice of warps per row has, with a last
+# block that is not full
+@pytest.mark.parametrize("rows,d", [(2048, 264), (2049, 512), (2047, 1024), (2049, 1024), (2049, 1040), (3, 2048),
+                                    (767, 4096), (769, 3080), (2049, 5120), (2047, 6144),
+                                    (2049, 6152), (9, 8192)])
+def test_rmsnorm_forward_row_counts(rows, d):
+    x = torch.randn(rows, d, device="cuda", dtype=bf16)
+    w = (1 + 0.1 * torch.randn(d, device="cuda")).to(bf16)
+    y, rstd = ops.rmsnorm_fwd(x, w, 1e-5)
+    yr, rstdr = R.rmsnorm_fwd(x.double(), w.double(), 1e-5)
+    assert _rel(y, yr) < 3e-3 and _rel(rstd, rstdr) < 1e-6   # as in test_rmsnorm_row_lengths
+
+
+# rows and heads on both sides of where a row gets more threads; a row's heads in several batches
+@pytest.mark.parametrize("rows,heads", [(1, 3), (64, 80), (600, 41), (2050, 20), (4099, 9), (9000, 1),
+                                        (9000, 17)])
+@pytest.mark.parametrize("hd", [16, 64, 128, 512])
+def test_rope_row_and_head_counts(rows, heads, hd):
+    cos, sin = R.rope_tables(500, hd, 10000.0, device="cuda")
+    x = torch.randn(rows, heads * hd + 8, device="cuda", dtype=bf16)
+    y = x.clone()
+    ops.rope_(y, cos, sin, 500, heads, hd)
+    ref = R.rope(x[:, : heads * hd].float().reshape(rows, heads, hd), cos, sin, 500, False)
+    assert _rel(y[:, : heads * hd], ref.reshape(rows, -1)) < 3e-3
+    assert torch.equal(y[:, heads * hd:], x[:, heads * hd:])
+
+
+# several rows per block, with rows left over; a block's chunks that are no whole number of warps
+@pytest.mark.parametrize("rows,F", [(300, 24), (1001, 120), (77, 2040), (513, 1000)])
+def test_swiglu_short_rows(rows, F):
+    gu = torch.randn(rows, 2 * F, device="cuda", dtype=bf16)
+    dh = torch.randn(rows, F, device="cuda", dtype=bf16)
+    assert _rel(ops.swiglu_fwd(gu), R.swiglu_fwd(gu)) < 3e-3
+    assert _rel(ops.swiglu_bwd(gu, dh), R.swiglu_bwd(gu, dh)) < 3e-3
+
+
+@pytest.mark.parametrize("rows,d", [(301, 64), (77, 2040)])
+def test_embedding_bwd_short_rows(rows, d):
+    ids = torch.randperm(400, device="cuda")[:rows]
+    dout = torch.randn(rows, d, device="cuda", dtype=bf16)
+    dt = torch.zeros(400, d, device="cuda", dtype=bf16)
+    ops.embedding_bwd_(dout, ids, dt)
+    ref = torch.zeros_like(dt)
+    ref[ids] = dout
+    assert torch.equal(dt, ref)
+
+
+@pytest.mark.parametrize("rows,V", [(512, 6144), (513, 6152), (511, 6144), (600, 16384), (600, 16396),
+                                    (5, 65535), (5, 65536)])
+def test_cross_entropy_block_sizes(rows, V):
+    ld = (V + 15) // 8 * 8
+    wide = (3 * torch.randn(rows, ld, device="cuda")).to(bf16)
+    tg = torch.randint(0, V, (rows,), device="cuda")
+    tg[:2] = torch.tensor([0, V - 1])
+    lr, gr = R.cross_entropy(wide[:, :V], tg, 0.25)
+    loss = ops.cross_entropy_(wide[:, :V], tg, 0.25)
+    assert torch.allclose(loss, lr, atol=2e-4, rtol=1e-4)   # as in test_cross_entropy_vocabularies
+    assert _rel(wide[:, :V], gr) < 3e-3
