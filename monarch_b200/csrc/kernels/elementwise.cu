@@ -159,7 +159,7 @@ constexpr int RMS_BWD_MAX_STAGES = 8;
 // A copy that does not land within the wait's limit is reported through the status word, and the
 // block's rows from there on and the weight gradient become NaN (the entry point without a status
 // word has only that).  Every thread still walks through all rows: none is missing at a barrier.
-// 8192x4096 with dres: 84.6 -> 48.2 us, 8192x5120: 245 -> 66 us, 8192x2048: 49.9 -> 34.8 us.
+// 8192x4096 with dres: 82.8 -> 48.2 us, 8192x5120: 239 -> 66 us, 8192x2048: 49.9 -> 34.8 us.
 template <int NT, int NCH, bool RES>
 __global__ void __launch_bounds__(NT, 1024 / (NT * NCH))
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -473,12 +473,13 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
 // Rows on grid.x, 8-column chunks on grid.y: no division per thread (a 64-bit one by F/8 cost
 // the forward a fifth of its time: 8192x14336 133.6 -> 113 us, backward 181 -> 178 us).  A block
 // takes several rows of fewer than 256 chunks.
+template <bool SHORT>   // several rows per block (their index costs the long ones 1 %)
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                   __nv_bfloat16* __restrict__ h, int rows, int F) {
   dep_wait();
-  const size_t row = (size_t)blockIdx.x * blockDim.y + threadIdx.y;
+  const size_t row = SHORT ? (size_t)blockIdx.x * blockDim.y + threadIdx.y : blockIdx.x;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (c >= F || row >= (size_t)rows) return;
+  if (c >= F || (SHORT && row >= (size_t)rows)) return;
   float g[8], u[8], o[8];
   load8(gu + row * 2 * F + c, g);
   load8(gu + row * 2 * F + F + c, u);
@@ -487,13 +488,14 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
   store8(h + row * F + c, o);
 }
 
+template <bool SHORT>
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                   const __nv_bfloat16* __restrict__ dh,
                                   __nv_bfloat16* __restrict__ dgu, int rows, int F) {
   dep_wait();
-  const size_t row = (size_t)blockIdx.x * blockDim.y + threadIdx.y;
+  const size_t row = SHORT ? (size_t)blockIdx.x * blockDim.y + threadIdx.y : blockIdx.x;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (c >= F || row >= (size_t)rows) return;
+  if (c >= F || (SHORT && row >= (size_t)rows)) return;
   float g[8], u[8], d[8], dg[8], du[8];
   load8(gu + row * 2 * F + c, g);
   load8(gu + row * 2 * F + F + c, u);
@@ -707,13 +709,14 @@ __global__ void embedding_fwd_kernel(const __nv_bfloat16* __restrict__ table,
 }
 // 16 bytes per reduction (four bf16 pairs, each element rounded as a single addition would
 // be): 8192x2048 34.8 -> 10.4 us against one pair per reduction.
+template <bool SHORT>
 __global__ void embedding_bwd_vec_kernel(const __nv_bfloat16* __restrict__ dout,
                                          const int64_t* __restrict__ ids,
                                          __nv_bfloat16* __restrict__ dtable, int rows, int d) {
   dep_wait();
-  const size_t row = (size_t)blockIdx.x * blockDim.y + threadIdx.y;
+  const size_t row = SHORT ? (size_t)blockIdx.x * blockDim.y + threadIdx.y : blockIdx.x;
   const int c = (int)(blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (c >= d || row >= (size_t)rows) return;
+  if (c >= d || (SHORT && row >= (size_t)rows)) return;
   const int64_t id = ids[row];
   const uint4 g = *reinterpret_cast<const uint4*>(dout + row * d + c);
   asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dtable + id * d + c),
@@ -832,16 +835,17 @@ extern "C" int mb200_swiglu_fwd(const void* gu, void* h, int rows, int F, void* 
   if (rows <= 0) return 0;
   if (F % 8 || F <= 0) return 1001;
   const dim3 b = row_block(F / 8);
-  return (int)launch_dep(swiglu_fwd_kernel, row_grid(rows, F / 8, b), b, 0, ST(stream), CBF(gu),
-                         BF(h), rows, F);
+  return (int)launch_dep(b.y > 1 ? swiglu_fwd_kernel<true> : swiglu_fwd_kernel<false>,
+                         row_grid(rows, F / 8, b), b, 0, ST(stream), CBF(gu), BF(h), rows, F);
 }
 extern "C" int mb200_swiglu_bwd(const void* gu, const void* dh, void* dgu, int rows, int F,
                                 void* stream) {
   if (rows <= 0) return 0;
   if (F % 8 || F <= 0) return 1001;
   const dim3 b = row_block(F / 8);
-  return (int)launch_dep(swiglu_bwd_kernel, row_grid(rows, F / 8, b), b, 0, ST(stream), CBF(gu),
-                         CBF(dh), BF(dgu), rows, F);
+  return (int)launch_dep(b.y > 1 ? swiglu_bwd_kernel<true> : swiglu_bwd_kernel<false>,
+                         row_grid(rows, F / 8, b), b, 0, ST(stream), CBF(gu), CBF(dh), BF(dgu), rows,
+                         F);
 }
 
 extern "C" int mb200_cross_entropy_fwd_bwd(void* logits, const int64_t* targets, float* loss_rows,
@@ -886,8 +890,10 @@ extern "C" int mb200_embedding_bwd(const void* dout, const int64_t* ids, void* d
   if (d % 2 || d <= 0) return 1001;
   if (d % 8 == 0 && aligned16(dout) && aligned16(dtable)) {
     const dim3 b = row_block(d / 8);
-    return (int)launch_dep(embedding_bwd_vec_kernel, row_grid(rows, d / 8, b), b, 0, ST(stream),
-                           CBF(dout), ids, BF(dtable), rows, d);
+    return (int)launch_dep(b.y > 1 ? embedding_bwd_vec_kernel<true>
+                                   : embedding_bwd_vec_kernel<false>,
+                           row_grid(rows, d / 8, b), b, 0, ST(stream), CBF(dout), ids, BF(dtable),
+                           rows, d);
   }
   const long long total = (long long)rows * (d / 2);
   return (int)launch_dep(embedding_bwd_kernel, blocks_for(total, 256), 256, 0, ST(stream),
