@@ -426,16 +426,18 @@ static int g_gemm_impl = 2;
 // 54.5 -> 55.1, 128x128 67.0 -> 68.7; 2048^3 128x256 17.5 -> 15.2, pair 18.0 -> 16.6;
 // 1000x2048x3072 128x128 16.1 -> 14.4, pair 23.6 -> 21.2; 200x768x256 128x64 4.4 -> 4.7, pair
 // 8.4 -> 9.0; 64x4096x4096 128x128 in 4 parts 10.3 -> 10.1, 128x64 in 2 parts 10.8 -> 11.1;
-// 1704x13136x160 pair 29.2 -> 27.8, 128x256 28.5 -> 23.2.
+// 3928x10808x38 pair 41.5 -> 47.8, 128x256 29.1 -> 35.7, 128x64 35.6 -> 43.2.
 //
-// Rows of A, B or C that do not start on 128-byte lines cost the single CTAs more than the pair,
-// whose tiles share fewer lines with their neighbours: kUnaligned, for 128x256 always, for the
-// narrower ones once there is more than one wave.  2944x408x5432 128x256 53.4 us, pair 41.3;
+// Rows of A, B or C that do not start on 128-byte lines make a step of the single CTAs longer by
+// `unaligned`, for 128x256 always, for the narrower ones once there is more than one wave (the
+// pair's tiles share fewer lines with their neighbours): 2944x408x5432 128x256 53.4 us, pair 41.3;
 // 352x13448x1352 128x128 31.7 and 28.8; 6968x984x912 27.1 and 24.6; but 3072x2048x1000 with both
-// operands along 3072 and 2048 128x128 15.8 and 17.8.  Over 44 shapes in four layouts the choice
-// takes 0.8 % more than the best tile; without e and kUnaligned 3.4 %, and 26 of the 144
-// products that no split takes were slower than the pair, by up to 17 %.
-constexpr float kUnaligned = 1.15f;
+// operands along 3072 and 2048 128x128 15.8 and 17.8.
+//
+// Over 243 products without a split (K from 1 to 15768, four layouts; e and `unaligned` are
+// fitted to them, t0 and c are from aligned ones) the choice takes 0.6 % more than the best tile
+// and 3 are slower than the pair by over 1 %, by at most 5 %; without e and `unaligned` 3.5 % more,
+// 34 slower than the pair, by up to 17 %.
 struct GemmPlan {
   int bn;      // 0: the CTA pair's 256x256 tile, else the columns of a single CTA's 128-row tile
   int split;   // CTAs of a cluster that share a tile along K
@@ -460,17 +462,17 @@ static GemmPlan gemm_plan(int M, int N, int K, bool aligned) {
     const float step = c * iters;
     return t0 + (waves - 1) * (step > e ? step : e) + step;
   };
-  float t = 0.98f * estimate(7.0f, 0.345f, 5.3f, div(div(M, G2_BM) * div(N, G2_BN), sms / 2));
-  struct { int bn; float t0, c, e, t_split[3]; } const kinds[] = {
-      {256, 5.2f, 0.385f, 4.6f, {0.f, 0.f, 0.f}},
-      {128, 4.3f, 0.245f, 3.0f, {1.05f, 2.1f, 3.2f}},   // splits of 2, 4, 8
-      {64, 3.6f, 0.200f, 2.2f, {0.8f, 1.5f, 2.3f}},
+  // an estimate within 2 % of the pair's goes to the pair (6136x5992x656 66.9, 128x256 83.4 us)
+  float t = 0.98f * estimate(7.0f, 0.345f, 3.8f, div(div(M, G2_BM) * div(N, G2_BN), sms / 2));
+  struct { int bn; float t0, c, e, unaligned, t_split[3]; } const kinds[] = {
+      {256, 5.2f, 0.385f, 2.6f, 1.4f, {0.f, 0.f, 0.f}},
+      {128, 4.3f, 0.245f, 1.75f, 1.55f, {1.05f, 2.1f, 3.2f}},   // splits of 2, 4, 8
+      {64, 3.6f, 0.200f, 0.9f, 1.55f, {0.8f, 1.5f, 2.3f}},
   };
   for (const auto& k : kinds) {
     const long long tiles = div(M, GEMM_BM) * div(N, k.bn);
-    // an estimate within 2 % of the pair's goes to the pair (6136x5992x656 66.9, 128x256 83.4 us)
-    const float u = estimate(k.t0, k.c, k.e, div(tiles, sms)) *
-                    (aligned || (k.bn != 256 && tiles <= sms) ? 1.f : kUnaligned);
+    const bool slow = !aligned && (k.bn == 256 || tiles > sms);
+    const float u = estimate(k.t0, k.c * (slow ? k.unaligned : 1.f), k.e, div(tiles, sms));
     if (u < t) t = u, best = {k.bn, 1};
     if (k.bn == 256) continue;
     for (int i = 0; i < 3; ++i) {
