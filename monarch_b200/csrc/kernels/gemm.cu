@@ -45,17 +45,18 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
-int sm_count() {
+static int sm_count(int dev) {
   static PerDevice<int> known;
-  int* n = known.here();
+  int* n = known.at(dev);
   int now = n ? *n : 0;
   if (!now) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&now, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&now, cudaDevAttrMultiProcessorCount, dev < 0 ? 0 : dev);
     if (n) *n = now;
   }
   return now;
+}
+int sm_count() {
+  return sm_count(current_device());
 }
 
 template <bool A_MN, bool B_MN, int BN, int EPI>
@@ -68,10 +69,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 
 template <bool A_MN, bool B_MN, int BN, int EPI = kEpiStore>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
-                  cudaStream_t st) {
+                  cudaStream_t st, int dev) {
   static PerDevice<int> smem_ok;
   if (const cudaError_t e =
-          allow_smem(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>, GemmTile<BN>::kSmemBytes, smem_ok))
+          allow_smem(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>, GemmTile<BN>::kSmemBytes, smem_ok, dev))
     return (int)e;
   return (int)launch_dep(gemm_bf16_kernel<A_MN, B_MN, BN, EPI>, grid, GEMM_THREADS,
                          GemmTile<BN>::kSmemBytes, st, ta, tb, p);
@@ -98,15 +99,15 @@ int make_gemm_tmaps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void*
 
 template <int BN>
 static int launch_gemm_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                          int a_mn, int b_mn, int grid, cudaStream_t st) {
-  if (a_mn && b_mn) return launch<true, true, BN>(ta, tb, p, grid, st);
-  if (a_mn) return launch<true, false, BN>(ta, tb, p, grid, st);
-  if (b_mn) return launch<false, true, BN>(ta, tb, p, grid, st);
-  return launch<false, false, BN>(ta, tb, p, grid, st);
+                          int a_mn, int b_mn, int grid, cudaStream_t st, int dev) {
+  if (a_mn && b_mn) return launch<true, true, BN>(ta, tb, p, grid, st, dev);
+  if (a_mn) return launch<true, false, BN>(ta, tb, p, grid, st, dev);
+  if (b_mn) return launch<false, true, BN>(ta, tb, p, grid, st, dev);
+  return launch<false, false, BN>(ta, tb, p, grid, st, dev);
 }
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int a_mn,
                 int b_mn, int grid, cudaStream_t st) {
-  return launch_gemm_bn<GEMM_BN>(ta, tb, p, a_mn, b_mn, grid, st);
+  return launch_gemm_bn<GEMM_BN>(ta, tb, p, a_mn, b_mn, grid, st, current_device());
 }
 
 // ------------------------------------------------------------------- split over K
@@ -284,18 +285,18 @@ __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 
 // Number of clusters of SPLIT CTAs that can be resident at once; 0 when there is no answer.
 template <bool A_MN, bool B_MN, int BN, int SPLIT>
-static int split_capacity() {
+static int split_capacity(int dev) {
   static PerDevice<int> known;   // capacity + 1
-  int* cap = known.here();
+  int* cap = known.at(dev);
   if (cap && *cap) return *cap - 1;
   static PerDevice<int> smem_ok;
-  if (allow_smem(gemm_split_kernel<A_MN, B_MN, BN, SPLIT>, GemmTile<BN>::kSmemBytes, smem_ok) !=
-      cudaSuccess) {
+  if (allow_smem(gemm_split_kernel<A_MN, B_MN, BN, SPLIT>, GemmTile<BN>::kSmemBytes, smem_ok,
+                 dev) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(SPLIT * (sm_count() / SPLIT));
+  cfg.gridDim = dim3(SPLIT * (sm_count(dev) / SPLIT));
   cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = GemmTile<BN>::kSmemBytes;
   cudaLaunchAttribute attr[1];
@@ -317,25 +318,25 @@ static int split_capacity() {
 
 template <bool A_MN, bool B_MN, int BN, int SPLIT>
 static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                        int tiles, cudaStream_t st) {
-  if (split_capacity<A_MN, B_MN, BN, SPLIT>() <= 0) return 1002;
+                        int tiles, cudaStream_t st, int dev) {
+  if (split_capacity<A_MN, B_MN, BN, SPLIT>(dev) <= 0) return 1002;
   return (int)launch_dep(gemm_split_kernel<A_MN, B_MN, BN, SPLIT>, tiles * SPLIT, GEMM_THREADS,
                          GemmTile<BN>::kSmemBytes, st, ta, tb, p);
 }
 template <int BN, int SPLIT>
 static int launch_split_ab(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                           int a_mn, int b_mn, int tiles, cudaStream_t st) {
-  if (a_mn && b_mn) return launch_split<true, true, BN, SPLIT>(ta, tb, p, tiles, st);
-  if (a_mn) return launch_split<true, false, BN, SPLIT>(ta, tb, p, tiles, st);
-  if (b_mn) return launch_split<false, true, BN, SPLIT>(ta, tb, p, tiles, st);
-  return launch_split<false, false, BN, SPLIT>(ta, tb, p, tiles, st);
+                           int a_mn, int b_mn, int tiles, cudaStream_t st, int dev) {
+  if (a_mn && b_mn) return launch_split<true, true, BN, SPLIT>(ta, tb, p, tiles, st, dev);
+  if (a_mn) return launch_split<true, false, BN, SPLIT>(ta, tb, p, tiles, st, dev);
+  if (b_mn) return launch_split<false, true, BN, SPLIT>(ta, tb, p, tiles, st, dev);
+  return launch_split<false, false, BN, SPLIT>(ta, tb, p, tiles, st, dev);
 }
 template <int BN>
 static int launch_split_n(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                          int a_mn, int b_mn, int split, int tiles, cudaStream_t st) {
-  if (split == 8) return launch_split_ab<BN, 8>(ta, tb, p, a_mn, b_mn, tiles, st);
-  if (split == 4) return launch_split_ab<BN, 4>(ta, tb, p, a_mn, b_mn, tiles, st);
-  return launch_split_ab<BN, 2>(ta, tb, p, a_mn, b_mn, tiles, st);
+                          int a_mn, int b_mn, int split, int tiles, cudaStream_t st, int dev) {
+  if (split == 8) return launch_split_ab<BN, 8>(ta, tb, p, a_mn, b_mn, tiles, st, dev);
+  if (split == 4) return launch_split_ab<BN, 4>(ta, tb, p, a_mn, b_mn, tiles, st, dev);
+  return launch_split_ab<BN, 2>(ta, tb, p, a_mn, b_mn, tiles, st, dev);
 }
 
 // ------------------------------------------------------------------ CTA-pair variant
@@ -352,9 +353,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm2_threads(EPI), 
 template <bool A_MN, bool B_MN, int EPI>
 static int pair_capacity() {
   static PerDevice<int> known, smem_ok;
-  int* cap = known.here();
+  const int dev = current_device();
+  int* cap = known.at(dev);
   if (cap && *cap) return *cap;
-  if (allow_smem(gemm2_bf16_kernel<A_MN, B_MN, EPI>, G2_SMEM_BYTES, smem_ok) != cudaSuccess)
+  if (allow_smem(gemm2_bf16_kernel<A_MN, B_MN, EPI>, G2_SMEM_BYTES, smem_ok, dev) != cudaSuccess)
     return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (sm_count() / 2));
@@ -443,24 +445,24 @@ struct GemmPlan {
   int split;   // CTAs of a cluster that share a tile along K
 };
 // Clusters of `split` CTAs that run at once (they have to share a GPC: fewer than SMs / split).
-static int split_clusters(int bn, int split) {
+static int split_clusters(int bn, int split, int dev) {
   if (bn == 64)
-    return split == 2   ? split_capacity<false, false, 64, 2>()
-           : split == 4 ? split_capacity<false, false, 64, 4>()
-                        : split_capacity<false, false, 64, 8>();
-  return split == 2   ? split_capacity<false, false, 128, 2>()
-         : split == 4 ? split_capacity<false, false, 128, 4>()
-                      : split_capacity<false, false, 128, 8>();
+    return split == 2   ? split_capacity<false, false, 64, 2>(dev)
+           : split == 4 ? split_capacity<false, false, 64, 4>(dev)
+                        : split_capacity<false, false, 64, 8>(dev);
+  return split == 2   ? split_capacity<false, false, 128, 2>(dev)
+         : split == 4 ? split_capacity<false, false, 128, 4>(dev)
+                      : split_capacity<false, false, 128, 8>(dev);
 }
 // aligned: the leading dimensions of A, B and C are multiples of 64 elements
-static GemmPlan gemm_plan(int M, int N, int K, bool aligned) {
+static GemmPlan gemm_plan(int M, int N, int K, bool aligned, int dev) {
   const int iters = (K + GEMM_BK - 1) / GEMM_BK;
   const auto div = [](long long a, long long b) { return (a + b - 1) / b; };
-  const int sms = sm_count();
+  const int sms = sm_count(dev);
   GemmPlan best = {0, 1};
   const auto estimate = [&](float t0, float c, float e, long long waves) {
-    const float step = c * iters;
-    return t0 + (waves - 1) * (step > e ? step : e) + step;
+    const float steps = c * iters;
+    return t0 + (waves - 1) * (steps > e ? steps : e) + steps;
   };
   // an estimate within 2 % of the pair's goes to the pair (6136x5992x656 66.9, 128x256 83.4 us)
   float t = 0.98f * estimate(7.0f, 0.345f, 3.8f, div(div(M, G2_BM) * div(N, G2_BN), sms / 2));
@@ -478,7 +480,7 @@ static GemmPlan gemm_plan(int M, int N, int K, bool aligned) {
     for (int i = 0; i < 3; ++i) {
       const int split = 2 << i;
       // one wave only
-      if (tiles * split > sms || iters < 2 * split || tiles > split_clusters(k.bn, split)) break;
+      if (tiles * split > sms || iters < 2 * split || tiles > split_clusters(k.bn, split, dev)) break;
       const float v = k.t0 + k.t_split[i] + k.c * div(iters, split);
       if (v < t) t = v, best = {k.bn, split};
     }
@@ -509,7 +511,8 @@ extern "C" int mb200_gemm_bf16(const void* A, const void* B, void* C, const void
   p.n_blk_rot = 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CUtensorMap ta, tb;
-  const GemmPlan plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, ((lda | ldb | ldc) & 63) == 0)
+  const int dev = current_device();
+  const GemmPlan plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, ((lda | ldb | ldc) & 63) == 0, dev)
                                          : GemmPlan{GEMM_BN, 1};
   const int bn = plan.bn;
   if (bn == 0) {
@@ -520,12 +523,12 @@ extern "C" int mb200_gemm_bf16(const void* A, const void* B, void* C, const void
   if (r) return 1000 - r;
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + bn - 1) / bn);
   if (plan.split > 1)
-    return bn == 64 ? launch_split_n<64>(ta, tb, p, a_mn, b_mn, plan.split, tiles, st)
-                    : launch_split_n<128>(ta, tb, p, a_mn, b_mn, plan.split, tiles, st);
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  if (bn == 64) return launch_gemm_bn<64>(ta, tb, p, a_mn, b_mn, grid, st);
-  if (bn == 128) return launch_gemm_bn<128>(ta, tb, p, a_mn, b_mn, grid, st);
-  return launch_gemm(ta, tb, p, a_mn, b_mn, grid, st);
+    return bn == 64 ? launch_split_n<64>(ta, tb, p, a_mn, b_mn, plan.split, tiles, st, dev)
+                    : launch_split_n<128>(ta, tb, p, a_mn, b_mn, plan.split, tiles, st, dev);
+  const int sms = sm_count(dev), grid = tiles < sms ? tiles : sms;
+  if (bn == 64) return launch_gemm_bn<64>(ta, tb, p, a_mn, b_mn, grid, st, dev);
+  if (bn == 128) return launch_gemm_bn<128>(ta, tb, p, a_mn, b_mn, grid, st, dev);
+  return launch_gemm_bn<GEMM_BN>(ta, tb, p, a_mn, b_mn, grid, st, dev);
 }
 
 // ------------------------------------------------------- gated activation in the epilogue
@@ -557,16 +560,17 @@ constexpr int kGluSmallMaxK = 1024;   // longer products outlast the host's seco
 
 enum GluKind { kGluFwd, kGluFwdKeep, kGluBwd };
 // 1: CTA-pair tile, 0: small single-CTA tile, -1: two kernels.
-static int glu_tile(GluKind kind, int M, int N, int F, int K, bool aligned, GemmPlan* plan) {
-  *plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, aligned) : GemmPlan{128, 1};
+static int glu_tile(GluKind kind, int M, int N, int F, int K, bool aligned, int dev,
+                    GemmPlan* plan) {
+  *plan = g_gemm_impl == 2 ? gemm_plan(M, N, K, aligned, dev) : GemmPlan{128, 1};
   if (plan->split > 1) return -1;
   const auto div = [](int a, int b) { return (long long)(a + b - 1) / b; };
   if (plan->bn == 64 || plan->bn == 128) {
     if (kind == kGluBwd && plan->bn != 64) return -1;
-    return div(M, GEMM_BM) * div(F, 64) <= sm_count() && K <= kGluSmallMaxK ? 0 : -1;
+    return div(M, GEMM_BM) * div(F, 64) <= sm_count(dev) && K <= kGluSmallMaxK ? 0 : -1;
   }
   if (F % 128) return -1;
-  const long long tiles = div(M, G2_BM) * div(N, G2_BN), pairs = sm_count() / 2;
+  const long long tiles = div(M, G2_BM) * div(N, G2_BN), pairs = sm_count(dev) / 2;
   bool fuse;
   if (kind == kGluFwd)
     fuse = plan->bn == 0 || tiles > 8 * pairs;
@@ -585,8 +589,9 @@ extern "C" int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void
       ((reinterpret_cast<uintptr_t>(H) | reinterpret_cast<uintptr_t>(gu)) & 15))
     return 1001;
   GemmPlan plan;
+  const int dev = current_device();
   const int tile = glu_tile(keep_gu ? kGluFwdKeep : kGluFwd, M, 2 * F, F, K,
-                            ((lda | ldw | ldh | ld_gu) & 63) == 0, &plan);
+                            ((lda | ldw | ldh | ld_gu) & 63) == 0, dev, &plan);
   if (tile < 0) {
     if (!gu) return MB200_NOT_FUSED;
     const int rc = ld_gu == 2 * F && ldh == F
@@ -618,9 +623,9 @@ extern "C" int mb200_gemm_swiglu_fwd(const void* A, const void* W, void* H, void
   const int r = make_gemm_tmaps_bn(&ta, &tb, A, W, M, 2 * F, K, lda, ldw, 0, 0, 64);
   if (r) return 1000 - r;
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * (F / 64);
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  return gu ? launch<false, false, 128, kEpiSwigluFwdKeep>(ta, tb, p, grid, st)
-            : launch<false, false, 128, kEpiSwigluFwd>(ta, tb, p, grid, st);
+  const int sms = sm_count(dev), grid = tiles < sms ? tiles : sms;
+  return gu ? launch<false, false, 128, kEpiSwigluFwdKeep>(ta, tb, p, grid, st, dev)
+            : launch<false, false, 128, kEpiSwigluFwd>(ta, tb, p, grid, st, dev);
 }
 
 // dgu[M, 2F] = gradient of silu(gate) * up at gu for dh = A W (W [K, F] row-major), without
@@ -633,7 +638,8 @@ extern "C" int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* g
                                  reinterpret_cast<uintptr_t>(dgu)) & 15))
     return 1001;
   GemmPlan plan;
-  const int tile = glu_tile(kGluBwd, M, F, F, K, ((lda | ldw | ld_gu) & 63) == 0, &plan);
+  const int dev = current_device();
+  const int tile = glu_tile(kGluBwd, M, F, F, K, ((lda | ldw | ld_gu) & 63) == 0, dev, &plan);
   if (tile < 0) {
     if (!dh) return MB200_NOT_FUSED;
     const int rc = ld_gu == 2 * F ? mb200_gemm_bf16(A, W, dh, nullptr, M, F, K, lda, ldw, F, 0, 0, 1, 0,
@@ -660,14 +666,14 @@ extern "C" int mb200_gemm_swiglu_bwd(const void* A, const void* W, const void* g
   const int r = make_gemm_tmaps_bn(&ta, &tb, A, W, M, F, K, lda, ldw, 0, 1, 64);
   if (r) return 1000 - r;
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((F + 63) / 64);
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  return launch<false, true, 64, kEpiSwigluBwd>(ta, tb, p, grid, st);
+  const int sms = sm_count(dev), grid = tiles < sms ? tiles : sms;
+  return launch<false, true, 64, kEpiSwigluBwd>(ta, tb, p, grid, st, dev);
 }
 
 // The tile (columns; 0: the CTA pair's) and K split that a product takes.
 extern "C" int mb200_gemm_plan(int M, int N, int K, int lda, int ldb, int ldc, int* bn, int* split) {
   if (M <= 0 || N <= 0 || K <= 0) return 1001;
-  const GemmPlan plan = gemm_plan(M, N, K, ((lda | ldb | ldc) & 63) == 0);
+  const GemmPlan plan = gemm_plan(M, N, K, ((lda | ldb | ldc) & 63) == 0, current_device());
   *bn = plan.bn;
   *split = plan.split;
   return 0;

@@ -10,18 +10,20 @@ constexpr int kMaxDevices = 64;
 template <typename T>
 struct PerDevice {
   T v[kMaxDevices] = {};
-  // the current device's entry, or null when there is none to keep (nothing is remembered then)
-  T* here() {
-    int dev = 0;
-    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices ? &v[dev] : nullptr;
-  }
+  // the entry of device `dev`, or null when there is none to keep (nothing is remembered then)
+  T* at(int dev) { return dev >= 0 && dev < kMaxDevices ? &v[dev] : nullptr; }
 };
+static inline int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
 
-// Lets `kernel` use `bytes` of dynamic shared memory on the current device.  `done` is this
-// kernel's own; setting the attribute twice from two threads does no harm.
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device, which is `dev`.
+// `done` is this kernel's own; setting the attribute twice from two threads does no harm.
 template <typename F>
-static inline cudaError_t allow_smem(F* kernel, int bytes, PerDevice<int>& done) {
-  int* have = done.here();
+static inline cudaError_t allow_smem(F* kernel, int bytes, PerDevice<int>& done,
+                                     int dev = current_device()) {
+  int* have = done.at(dev);
   if (have && *have >= bytes) return cudaSuccess;
   const cudaError_t e =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
