@@ -146,10 +146,10 @@ def swiglu_bwd(gu, dh, out=None):
 
 
 _NOT_FUSED, _TWO_KERNELS = 1003, 1004   # MB200_NOT_FUSED, MB200_TWO_KERNELS
-
-
-def _check_glu(rc, what):
-    K.check(0 if rc == _TWO_KERNELS else rc, what, 2 if rc == _TWO_KERNELS else 1)
+# Rows x F for which the library most likely launches two kernels: more than one wave of small
+# tiles and less than pair tiles fuse for.  The matrix between the two is ready then; elsewhere
+# the library asks for it, a call of 2 us more.
+_LIKELY_TWO = (1 << 20, 1 << 23)
 
 
 def gemm_swiglu(a, w_gu, keep_gu=True):
@@ -162,15 +162,23 @@ def gemm_swiglu(a, w_gu, keep_gu=True):
         Kd = a.shape[1]
         assert w_gu.shape == (2 * F, Kd), (a.shape, w_gu.shape)
         h = torch.empty(T, F, dtype=bf16, device=a.device)
-        gu = torch.empty(T, 2 * F, dtype=bf16, device=a.device) if keep_gu else None
-        while True:
-            rc = K.lib().mb200_gemm_swiglu_fwd(
+        gu = None
+        if keep_gu or _LIKELY_TWO[0] <= T * F <= _LIKELY_TWO[1]:
+            gu = torch.empty(T, 2 * F, dtype=bf16, device=a.device)
+
+        def run(gu):
+            return K.lib().mb200_gemm_swiglu_fwd(
                 a.data_ptr(), w_gu.data_ptr(), h.data_ptr(), _p(gu), T, F, Kd, lda, ldw, F, 2 * F,
                 int(keep_gu), K.status_ptr(a), K.stream_ptr())
-            if rc != _NOT_FUSED:
-                break
+
+        rc = run(gu)
+        if rc == _NOT_FUSED:
             gu = torch.empty(T, 2 * F, dtype=bf16, device=a.device)
-        _check_glu(rc, "gemm_swiglu_fwd")
+            rc = run(gu)
+        if rc == _TWO_KERNELS:
+            K.check(0, "gemm_swiglu_fwd", 2)
+        else:
+            K.check(rc, "gemm_swiglu_fwd")
         return h, (gu if keep_gu else None)
     gu = gemm(a, w_gu)
     return swiglu_fwd(gu), (gu if keep_gu else None)
@@ -188,14 +196,22 @@ def gemm_swiglu_bwd(dy, w_down, gu):
         assert w_down.shape[0] == Kd and gu.shape == (T, 2 * F), (dy.shape, w_down.shape, gu.shape)
         dgu = torch.empty_like(gu)
         dh = None
-        while True:
-            rc = K.lib().mb200_gemm_swiglu_bwd(
+        if _LIKELY_TWO[0] <= T * F <= _LIKELY_TWO[1]:
+            dh = torch.empty(T, F, dtype=bf16, device=dy.device)
+
+        def run(dh):
+            return K.lib().mb200_gemm_swiglu_bwd(
                 dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(), _p(dh), T, F, Kd,
                 lda, ldw, 2 * F, K.status_ptr(dy), K.stream_ptr())
-            if rc != _NOT_FUSED:
-                break
+
+        rc = run(dh)
+        if rc == _NOT_FUSED:
             dh = torch.empty(T, F, dtype=bf16, device=dy.device)
-        _check_glu(rc, "gemm_swiglu_bwd")
+            rc = run(dh)
+        if rc == _TWO_KERNELS:
+            K.check(0, "gemm_swiglu_bwd", 2)
+        else:
+            K.check(rc, "gemm_swiglu_bwd")
         return dgu
     return swiglu_bwd(gu, gemm(dy, w_down, b_mn=True))
 
