@@ -355,12 +355,13 @@ class LlamaEngine:
     """
 
     def __init__(self, cfg: LlamaConfig, store, seq_len: int, checkpoint: bool = True,
-                 recompute_layers: Optional[int] = None, keep_residual: bool = False):
+                 recompute_layers: Optional[int] = None, keep_residual: Optional[bool] = None):
         """``checkpoint``: keep only each layer's input (and, with the attention kernels, its
         attention output) in the forward and recompute the rest in the backward.
         ``keep_residual`` (with both): also keep the residual stream behind the attention, 2
         more bytes per token and model-dim element of each recomputed layer, so that the
-        output projection is not run again.  ``recompute_layers`` (with ``checkpoint``):
+        output projection is not run again; None: when that is :attr:`KEEP_RESIDUAL_BYTES`
+        or less in all.  ``recompute_layers`` (with ``checkpoint``):
         how many of the layers, counted from the first, are treated that way; the remaining
         last layers keep all their activations (about 17 bytes per token per model-dim
         element each), trading spare HBM for one skipped forward per kept layer.  Default:
@@ -380,7 +381,16 @@ class LlamaEngine:
         # whose backward needs nothing else from the forward)
         self.keep_attention = checkpoint and ops.have_attention_kernel() and \
             torch.device(dev).type == "cuda"
-        self.keep_residual = keep_residual and self.keep_attention
+        self.keep_residual = keep_residual
+
+    # What keeping the residual streams may cost unasked: under 0.2 % of the device's memory, so
+    # that a model that only just fits keeps fitting.
+    KEEP_RESIDUAL_BYTES = 256 << 20
+
+    def _keeps_residual(self, T: int) -> bool:
+        if self.keep_residual is not None:
+            return self.keep_residual
+        return 2 * T * self.cfg.d * self.recompute_layers <= self.KEEP_RESIDUAL_BYTES
 
     # ------------------------------------------------------------------ layer forward
     def _attn_fwd(self, w: dict, x: torch.Tensor, B: int, S: int, keep: bool, attn_saved=None):
@@ -423,7 +433,7 @@ class LlamaEngine:
             return y, (sa, sm)
         actx = sa[3]
         if self.keep_attention and actx.lse is not None:
-            return y, (actx.o, actx.lse, x2 if self.keep_residual else None)
+            return y, (actx.o, actx.lse, x2 if self._keeps_residual(B * S) else None)
         return y, None
 
     def _mlp_bwd(self, w: dict, g: dict, sm, dy: torch.Tensor):

@@ -27,7 +27,7 @@ class Trainer:
                  micro_batch: int = 1, parallelism: str = "auto", device=None,
                  checkpoint: bool = True, lr: float = 3e-4, seed: int = 0,
                  comm: str = "fused", recompute_layers: Optional[int] = None,
-                 keep_residual: bool = False):
+                 keep_residual: Optional[bool] = None):
         self.cfg = PRESETS[model] if isinstance(model, str) else model
         self.seq_len = seq_len
         self.micro_batch = micro_batch

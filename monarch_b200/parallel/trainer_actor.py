@@ -85,7 +85,7 @@ class TrainerActor(Actor):
             self.trainer = Trainer(model, seq_len=seq, micro_batch=mb, parallelism=par,
                                    device=self.device, comm=comm,
                                    recompute_layers=s.get("recompute_layers"),
-                                   keep_residual=bool(s.get("keep_residual", False)),
+                                   keep_residual=s.get("keep_residual"),
                                    lr=float(s.get("lr", 3e-4)))
         self._pipeline = bool(m_pp)
         cfg = self.trainer.cfg

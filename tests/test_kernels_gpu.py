@@ -407,19 +407,28 @@ def test_checkpointing_keeps_the_residual_stream_only_when_asked(monkeypatch):
     tok = torch.randint(0, cfg.vocab, (1, T), device="cuda")
     held, grads, loss = {}, {}, ops.cross_entropy_
 
+    def requested():   # what was asked for, not the blocks that the allocator found for it
+        return torch.cuda.memory_stats()["requested_bytes.all.current"]
+
     def counted(*args):
-        held[keep] = torch.cuda.memory_allocated() - base
+        held[keep] = requested() - base
         return loss(*args)
 
     monkeypatch.setattr(ops, "cross_entropy_", counted)
-    for keep in (False, True):
+    cost = cfg.n_layers * T * cfg.d * 2
+    for keep, limit in ((False, None), (True, 0), (None, cost - 1), (None, cost)):
+        if limit is not None:
+            monkeypatch.setattr(LlamaEngine, "KEEP_RESIDUAL_BYTES", limit)
         st = LocalParamStore(ParamLayout(cfg), "cuda", seed=1)
-        eng = LlamaEngine(cfg, st, T, **({"keep_residual": True} if keep else {}))
-        base = torch.cuda.memory_allocated()
+        eng = LlamaEngine(cfg, st, T, keep_residual=keep)
+        keep = (keep, limit)
+        base = requested()
         eng.forward_backward(tok, tok)
         grads[keep] = [g.clone() for u in range(cfg.n_layers + 2) for g in st.unit_grads(u).values()]
-    assert held[True] - held[False] == cfg.n_layers * T * cfg.d * 2, held
-    assert all(torch.equal(a, b) for a, b in zip(grads[False][1:], grads[True][1:]))
+    no, yes = (False, None), (True, 0)
+    assert held[yes] - held[no] == cost, held
+    assert held[None, cost - 1] == held[no] and held[None, cost] == held[yes], held
+    assert all(torch.equal(a, b) for a, b in zip(grads[no][1:], grads[yes][1:]))
 
 
 # both sides of every limit in rows and width that the choice of warps per row has, with a last

@@ -79,7 +79,7 @@ def test_flops_per_token_counts_the_products_that_run(monkeypatch, checkpoint, k
     st = LocalParamStore(ParamLayout(cfg), "cpu", seed=0)
     eng = LlamaEngine(cfg, st, seq_len=16, checkpoint=checkpoint)
     # as with the attention kernels, whose output and log-sum-exp are kept
-    eng.keep_attention, eng.keep_residual = checkpoint, keep_residual
+    eng.keep_attention, eng.keep_residual = checkpoint, keep_residual and checkpoint
     attend = ops.attention_fwd
 
     def attention_fwd(*a, **kw):
