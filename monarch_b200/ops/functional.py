@@ -82,6 +82,9 @@ def rmsnorm_fwd(x, w, eps=1e-5):
     return y, rstd
 
 
+_rms_most_blocks: dict = {}   # device index -> mb200_rmsnorm_bwd_blocks of many rows
+
+
 def rmsnorm_bwd(dy, x, w, rstd, dw_out, accumulate=False, dres=None):
     """Returns dx (+ ``dres``); writes (or adds) the weight gradient into ``dw_out``."""
     rows, d = x.shape
@@ -95,9 +98,12 @@ def rmsnorm_bwd(dy, x, w, rstd, dw_out, accumulate=False, dres=None):
         return dx.to(x.dtype)
     dy = dy.contiguous()
     dx = torch.empty_like(x)
-    nb = K.lib().mb200_rmsnorm_bwd_blocks(rows)
+    dev = x.get_device()
+    most = _rms_most_blocks.get(dev)
+    if most is None:
+        most = _rms_most_blocks[dev] = K.lib().mb200_rmsnorm_bwd_blocks(1 << 30)
     # of this call alone: another stream's call may run between the two kernels that use it
-    part = torch.empty(nb * d, dtype=torch.float32, device=x.device)
+    part = torch.empty((rows if rows < most else most) * d, dtype=torch.float32, device=x.device)
     K.check(K.lib().mb200_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(),
                                       _p(dres), dx.data_ptr(), part.data_ptr(), dw_out.data_ptr(),
                                       int(accumulate), rows, d, K.status_ptr(x), K.stream_ptr()),

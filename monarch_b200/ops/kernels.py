@@ -20,6 +20,7 @@ _SO = Path(__file__).resolve().parent / ("_mb200_kernels_checked.so" if CHECKED
                                          else "_mb200_kernels.so")
 _lib: Optional[ctypes.CDLL] = None
 _status: dict[int, torch.Tensor] = {}
+_status_ptr: dict[int, int] = {}   # their addresses
 
 #: number of kernels of this library launched since import (bench.py reports the delta)
 launch_count = 0
@@ -197,8 +198,10 @@ def status_word(device: torch.device | int | None = None) -> torch.Tensor:
 
 def status_ptr(t: torch.Tensor) -> int:
     """Address of the status word of the device that holds ``t``."""
-    w = _status.get(t.get_device())
-    return (status_word(t.device) if w is None else w).data_ptr()
+    p = _status_ptr.get(t.get_device())
+    if p is None:
+        p = _status_ptr[t.get_device()] = status_word(t.device).data_ptr()
+    return p
 
 
 _STATUS_TEXT = {1: "mbarrier wait timed out inside a kernel",
