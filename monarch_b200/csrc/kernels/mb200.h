@@ -43,7 +43,8 @@ int mb200_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int ro
                       float eps, void* stream);
 // dx = d(loss)/dx (+ dres when given: the gradient arriving through the residual path);
 // dw_partial: fp32 scratch [nblocks, d]; dw: [d] bf16. nblocks is returned by
-// mb200_rmsnorm_bwd_blocks(rows).
+// mb200_rmsnorm_bwd_blocks(rows).  status: the device's status word, or null; a copy that never
+// lands is reported there, and leaves NaN in dw and in the rows of dx that it concerns.
 int mb200_rmsnorm_bwd_blocks(int rows);
 int mb200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
                       const void* dres, void* dx, float* dw_partial, void* dw, int dw_accumulate,
